@@ -134,9 +134,6 @@ cudaError_t run(const UQParams& p, const int32_t* pos_offset, float* o_part, flo
   UQLaunch x{};
   x.pos_offset = pos_offset;
   x.tree_mask = tree_mask;
-  x.k_first = 0;
-  x.k_total = p.K;
-  x.len_cut = 0;
   x.expire_id = forced_expire();
   x.status = status_ptr();
   if (!x.status) {
@@ -144,47 +141,32 @@ cudaError_t run(const UQParams& p, const int32_t* pos_offset, float* o_part, flo
     cudaGetDevice(&dev);
     return dev < 0 || dev >= kMaxDevices ? cudaErrorInvalidDevice : cudaErrorInitializationError;
   }
-  // More query rows than the tensor-core kernel takes in one launch (K * group > 64, up to the 128 of uq_block_m): the
-  // drafts are run as chunks of consecutive drafts, each a verify call of its own on the sequence cut after the chunk
-  // (see UQLaunch), sharing the caller's scratch one after the other.  A tree-masked call is chunked without the cut: its
-  // masks decide which of the caller's drafts a query sees, whichever chunk they belong to.
-  const int G = p.HQ / p.HKV;
-  const int per = G <= 64 ? 64 / G : 0;   // drafts per chunk
-  if (p.K * G > 64 && per >= 1 && forced_path() != 1) {
-    UQParams pc = p;
-    pc.K = per;
-    UQLaunch xc = x;
-    xc.G = G;
-    xc.rows = per * G;
-    if (uq_verify_tc_serves(pc, xc)) {
-      for (int k0 = 0; k0 < p.K; k0 += per) {
-        pc.K = std::min(per, p.K - k0);
-        xc.k_first = k0;
-        xc.len_cut = tree_mask ? 0 : p.K - k0 - pc.K;
-        UQPeerPush pp{};
-        if (push) {   // every chunk stores its rows into the peers' buffers; the last one raises the flags
-          pp = *push;
-          pp.raise = k0 + per >= p.K;
-        }
-        cudaError_t e = run_one(pc, xc, o_part, lse_part, s, push ? &pp : nullptr);
-        if (e != cudaSuccess) return e;
-      }
-      return cudaSuccess;
-    }
-  }
   return run_one(p, x, o_part, lse_part, s, push);
 }
 
 // One launch of a verify kernel and its combine; x carries the caller's pointers and the draft chunk.
 cudaError_t run_one(const UQParams& p, UQLaunch x, float* o_part, float* lse_part, cudaStream_t s, const UQPeerPush* push) {
   x.G = p.HQ / p.HKV;
+  x.chunks = 1;
+  x.per = p.K;
   x.rows = p.K * x.G;
   x.BM = uq_block_m(p.K, p.HQ, p.HKV);
   // NVFP4 (reference cuda/uq_decode.cu:604,384): k_ts is folded into the softmax scale, v_ts multiplies the output
   x.sc2 = p.sm_scale * (p.fmt == 1 ? p.k_ts : 1.f) * 1.4426950408889634f;
   x.out_scale = p.fmt == 1 ? p.v_ts : 1.f;
   const int forced = forced_path();
-  bool tc = forced != 1 && uq_verify_tc_serves(p, x);
+  // More query rows than the tensor-core kernel's tile takes (up to the 128 of uq_block_m): the drafts run as two chunks of one
+  // launch.  As two launches, one after the other in the same scratch, start-up, combine and an underfilled chip were paid
+  // twice: B=4, 8 K tokens, 16 drafts at a group of 8 took 61 us, 45 in one launch.
+  UQLaunch xc = x;
+  if (x.rows > 64 && x.G <= 64) {
+    const int fit = 64 / x.G;
+    xc.chunks = (p.K + fit - 1) / fit;
+    xc.per = (p.K + xc.chunks - 1) / xc.chunks;
+    xc.rows = xc.per * x.G;
+  }
+  bool tc = forced != 1 && uq_verify_tc_serves(p, xc);
+  if (tc) x = xc;
   if (forced == 2 && !tc) return cudaErrorInvalidValue;
   cudaError_t e;
   const bool timed = t_ev_before && t_ev_after;

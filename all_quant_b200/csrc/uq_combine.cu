@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(128) uq_combine_kernel(const UQParams p, const
   const int h = row % p.HQ, j = (row / p.HQ) % p.K, b = row / (p.HQ * p.K);
   const int hk = h / x.G, r = j * x.G + (h % x.G);
   const int D = p.D;
-  const size_t orow = uq_draft_row(x, b, j) * p.HQ + h;   // the row of the caller's [B, K, HQ] arrays (a chunk of drafts writes its own rows)
+  const size_t orow = uq_draft_row(p, b, j) * p.HQ + h;
   const size_t slot0 = uq_slot(p, b, hk, 0);
   // The slots' log-sum-exps are read lane-parallel (slot s by lane s mod 32: up to four per lane for nsplit <= 128), so the
   // row's maximum, weights and denominator cost a few loads instead of a serial chain of nsplit of them.

@@ -431,7 +431,7 @@ UQ_DEV float warp_fold(float* v, int lane) {
 // Which of the rows r0 .. r0 + n - 1 (row = draft j * G + head of the group) see draft token td of sequence b: bit i = row
 // r0 + i.  Out of line: it runs only in the one or two tiles of an item that hold the draft positions, and inlined it costs
 // the common tile registers.
-// (j_first: the caller's number of this launch's draft 0, K the caller's draft count, when a tree-masked call runs as chunks.)
+// (j_first: the first draft of the work item's chunk.)
 __device__ __noinline__ uint32_t draft_rows(const int32_t* tree_mask, int K, int b, int td, int r0, int n, int rows, int G, int j_first) {
   uint32_t m = 0u;
   for (int i = 0; i < n; i++) {
@@ -445,7 +445,8 @@ __device__ __noinline__ uint32_t draft_rows(const int32_t* tree_mask, int K, int
 
 // ---------------------------------------------------------------------------------------------- layout
 struct Seg {
-  int b, hk, t0, t1;   // tiles [t0, t1) of item (b, hk)
+  int b, hk, t0, t1;   // tiles [t0, t1) of item (b, hk, ch)
+  int ch;              // chunk of drafts
   int slot;            // partial slot of this segment
   int nseg;            // slots the item uses (valid when t0 == 0)
   int ntiles;          // tiles of the whole item
@@ -586,11 +587,11 @@ UQ_DEV int small_quotient(int n, int d) {
 
 struct Walker {
   const int* prefix;   // prefix[b] = weighted units of sequences < b (one kv head): tiles + kSegW per non-empty sequence
-  int B, HKV, nitems, total, chunk, per_item, kSegW;
+  int B, NI, chunks, nitems, total, chunk, per_item, kSegW;   // NI = items of one sequence: kv heads x chunks of drafts, a head's chunks next to each other (they read the same keys)
   int pos, end, it, cta;
 
-  UQ_DEV void init(const int* pre, int B_, int HKV_, int ns_eff, int chunk_min, int seg_w) {
-    prefix = pre; B = B_; HKV = HKV_; nitems = B * HKV; total = HKV * pre[B]; kSegW = seg_w;
+  UQ_DEV void init(const int* pre, int B_, int HKV_, int chunks_, int ns_eff, int chunk_min, int seg_w) {
+    prefix = pre; B = B_; chunks = chunks_; NI = HKV_ * chunks_; nitems = B * NI; total = NI * pre[B]; kSegW = seg_w;
     cta = blockIdx.x;
     per_item = ns_eff < 2;
     if (per_item) { it = cta - (int)gridDim.x; pos = end = 0; chunk = 1; return; }
@@ -601,18 +602,19 @@ struct Walker {
     end = min(pos + chunk, total);
     it = 0;
   }
-  UQ_DEV int item_tiles(int item) const { const int b = item / HKV; return max(prefix[b + 1] - prefix[b] - kSegW, 0); }
+  UQ_DEV void set_item(Seg& s, int i) const { if (chunks == 1) { s.hk = i; s.ch = 0; } else { s.hk = i / chunks; s.ch = i - s.hk * chunks; } }
+  UQ_DEV int item_tiles(int item) const { const int b = item / NI; return max(prefix[b + 1] - prefix[b] - kSegW, 0); }
   // Past the listed segments (out of line, like next(): the roles' loops should not carry this code or its registers)
-  __device__ __noinline__ bool next_after(Seg& s, const SegList* L, bool& walking, const int* pre, int B_, int HKV_, int ns_eff, int chunk_min, int seg_w) {
+  __device__ __noinline__ bool next_after(Seg& s, const SegList* L, bool& walking, const int* pre, int B_, int HKV_, int chunks_, int ns_eff, int chunk_min, int seg_w) {
     if (!walking) {
-      init(pre, B_, HKV_, ns_eff, chunk_min, seg_w);
+      init(pre, B_, HKV_, chunks_, ns_eff, chunk_min, seg_w);
       if (per_item) it = L->it_after; else pos = min(L->pos_after, end);
       walking = true;
     }
     return next(s);
   }
   // The same walk as next(), done by one warp in one step: lane j takes the j-th candidate item from the chunk's start
-  // (its item index is known without the items before it: unit position of item (b, hk) = HKV * prefix[b] + hk * width of b),
+  // (its item index is known without the items before it: unit position of item (b, hk) = NI * prefix[b] + hk * width of b),
   // the lanes whose item has tiles in the chunk are the segments, in lane order.  Called after init() by all 32 lanes.
   UQ_DEV void list(SegList* L, int lane) {
     Seg s;
@@ -622,27 +624,27 @@ struct Walker {
       beyond = item >= nitems;
       if (!beyond) {
         const int n = item_tiles(item);
-        if (n > 0) { s.b = item / HKV; s.hk = item - s.b * HKV; s.t0 = 0; s.t1 = n; s.slot = 0; s.nseg = 1; s.ntiles = n; valid = true; }
+        if (n > 0) { s.b = item / NI; set_item(s, item - s.b * NI); s.t0 = 0; s.t1 = n; s.slot = 0; s.nseg = 1; s.ntiles = n; valid = true; }
       }
     } else if (pos < end) {
-      int lo = 0, hi = B;                 // sequence containing unit `pos`: largest b with HKV * prefix[b] <= pos
+      int lo = 0, hi = B;                 // sequence containing unit `pos`: largest b with NI * prefix[b] <= pos
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (HKV * prefix[mid] <= pos) lo = mid; else hi = mid;
+        if (NI * prefix[mid] <= pos) lo = mid; else hi = mid;
       }
       const int nv0 = prefix[lo + 1] - prefix[lo];
-      const int item = lo * HKV + small_quotient(pos - HKV * prefix[lo], nv0) + lane;
-      const int b = small_quotient(item, HKV), hk = item - b * HKV;
+      const int item = lo * NI + small_quotient(pos - NI * prefix[lo], nv0) + lane;
+      const int b = small_quotient(item, NI), hk = item - b * NI;
       beyond = b >= B;
       if (!beyond) {
         const int nv = prefix[b + 1] - prefix[b], n = nv - kSegW;
-        const int start = HKV * prefix[b] + hk * nv, first = start + kSegW;
+        const int start = NI * prefix[b] + hk * nv, first = start + kSegW;
         beyond = start >= end;
         if (!beyond && nv > 0) {
           const int t0 = max(pos, first) - first, t1 = min(first + n, end) - first;
           if (t1 > t0) {
             const int c0 = small_quotient(first, chunk);
-            s.b = b; s.hk = hk; s.ntiles = n; s.t0 = t0; s.t1 = t1; s.slot = cta - c0;
+            s.b = b; set_item(s, hk); s.ntiles = n; s.t0 = t0; s.t1 = t1; s.slot = cta - c0;
             s.nseg = small_quotient(first + n - 1, chunk) - c0 + 1;
             valid = true;
           }
@@ -660,25 +662,25 @@ struct Walker {
       for (it += (int)gridDim.x; it < nitems; it += (int)gridDim.x) {
         const int n = item_tiles(it);
         if (n == 0) continue;
-        s.b = it / HKV; s.hk = it % HKV; s.t0 = 0; s.t1 = n; s.slot = 0; s.nseg = 1; s.ntiles = n;
+        s.b = it / NI; set_item(s, it % NI); s.t0 = 0; s.t1 = n; s.slot = 0; s.nseg = 1; s.ntiles = n;
         return true;
       }
       return false;
     }
     while (pos < end) {
-      // sequence containing unit `pos`: largest b with HKV * prefix[b] <= pos
+      // sequence containing unit `pos`: largest b with NI * prefix[b] <= pos
       int lo = 0, hi = B;
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (HKV * prefix[mid] <= pos) lo = mid; else hi = mid;
+        if (NI * prefix[mid] <= pos) lo = mid; else hi = mid;
       }
-      const int nv = prefix[lo + 1] - prefix[lo];   // > 0 because pos < HKV * prefix[lo + 1]
+      const int nv = prefix[lo + 1] - prefix[lo];   // > 0 because pos < NI * prefix[lo + 1]
       const int n = nv - kSegW;
-      const int hk = (pos - HKV * prefix[lo]) / nv;
-      const int first = HKV * prefix[lo] + hk * nv + kSegW;   // unit of the item's tile 0 (the kSegW units before it are the start-up weight)
+      const int hk = (pos - NI * prefix[lo]) / nv;
+      const int first = NI * prefix[lo] + hk * nv + kSegW;   // unit of the item's tile 0 (the kSegW units before it are the start-up weight)
       const int t0 = max(pos, first) - first, t1 = min(first + n, end) - first;
       if (t1 > t0) {
-        s.b = lo; s.hk = hk; s.ntiles = n; s.t0 = t0; s.t1 = t1;
+        s.b = lo; set_item(s, hk); s.ntiles = n; s.t0 = t0; s.t1 = t1;
         const int c0 = first / chunk;   // the CTA of the item's tile 0 writes slot 0
         s.slot = cta - c0;
         s.nseg = (first + n - 1) / chunk - c0 + 1;
@@ -786,7 +788,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   if (warp == 0) {   // the CTA's segments, once, for every role (the walker's struct lives in registers here)
     __syncwarp();
     Walker w0;
-    w0.init(prefix, p.B, p.HKV, x.ns_eff, prm.chunk_min, seg_weight(NT));
+    w0.init(prefix, p.B, p.HKV, x.chunks, x.ns_eff, prm.chunk_min, seg_weight(NT));
     w0.list(seglist, lane);
   }
   if (warp == kWarpMma) {
@@ -800,7 +802,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   UQ_TRACE_CTA_T(1)
 
   Walker wk;
-  const int G = x.G, rows = x.rows;
+  const int G = x.G;
   Seg sg;
   // Two passes over the CTA's segments.  The first takes every segment on the quick path: the softmax threads fix each
   // row's reference at the segment's first tile and afterwards only watch for a score or a V scale that no longer fits the
@@ -819,7 +821,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   auto next_seg = [&](Seg& s) -> bool {
     if (seg_at < seglist->n) { s = seglist->seg[seg_at++]; return true; }
     if (!seglist->more) return false;
-    return wk.next_after(s, seglist, walking, prefix, p.B, p.HKV, x.ns_eff, prm.chunk_min, seg_weight(NT));
+    return wk.next_after(s, seglist, walking, prefix, p.B, p.HKV, x.chunks, x.ns_eff, prm.chunk_min, seg_weight(NT));
   };
   int ord = -1;                    // ordinal of the segment in the CTA's list
   // does this pass run segment `ord`?  (pass 1: the marked ones)
@@ -1179,8 +1181,9 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
     // items without a single key: nobody computes them, their slots must read as empty
     for (int it = blockIdx.x; pass == 0 && it < p.B * p.HKV; it += gridDim.x) {
       { const int b = it / p.HKV; if (prefix[b + 1] - prefix[b] != 0) continue; }   // (an item with keys has tiles + the start-up weight)
-      for (int i = st; i < x.ns_eff * rows; i += kSm)
-        p.ml[uq_slot(p, it / p.HKV, it % p.HKV, i / rows) * x.BM + i % rows] = -INFINITY;
+      const int all = p.K * G;   // every chunk's rows
+      for (int i = st; i < x.ns_eff * all; i += kSm)
+        p.ml[uq_slot(p, it / p.HKV, it % p.HKV, i / all) * x.BM + i % all] = -INFINITY;
     }
     while (ok && next_seg(sg)) {
       if (!take()) continue;
@@ -1188,10 +1191,9 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
       const bool careful = pass == 1 || ord >= 32 * kRedoWords;
       int off;
       const int n_loc = uq_n_local(p, x, sg.b, &off);
-      const int n_glob = uq_seq_len(p, x, sg.b);
-      // draft positions counted back from the end: this launch's own drafts, or, for a chunk of a tree-masked call (which
-      // is not cut: any query may be given any draft by its mask), all of the caller's
-      const int Kq = x.tree_mask ? x.k_total : p.K, j_first = x.tree_mask ? x.k_first : 0;
+      const int n_glob = p.seq_lens[sg.b];
+      // this item's drafts j_first .. and their query rows; the masked positions are the call's K last ones in every chunk
+      const int j_first = sg.ch * x.per, rows = min(x.per, p.K - j_first) * G, row_off = j_first * G;
       // ---- query tile in fp16, natural channel order, 128-byte swizzle, two 64-channel halves.  The tile is scaled by a
       // power of two so that its largest magnitude lies in [1, 2) (bf16 queries of any range fit fp16 this way; entries
       // below 2^-24 of the largest vanish); the power goes back into the softmax scale.
@@ -1208,7 +1210,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < 16; j++) qv[j] = 0.f;
           if (i < kItems && n < rows) {
-            const uint4* src = reinterpret_cast<const uint4*>(qg + ((uq_draft_row(x, sg.b, n / G)) * p.HQ + sg.hk * G + n % G) * D) + 2 * a;
+            const uint4* src = reinterpret_cast<const uint4*>(qg + (uq_draft_row(p, sg.b, j_first + n / G) * p.HQ + sg.hk * G + n % G) * D) + 2 * a;
             const uint4 v0 = __ldg(src), v1 = __ldg(src + 1);
             const uint32_t w8[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
@@ -1266,7 +1268,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         uint32_t amax = 0;   // bf16 magnitudes compare as integers
         for (int i = st; i < rows * (D / 8); i += kSm) {
           const int n = i / (D / 8), a = i % (D / 8);
-          const uint4 v = __ldg(reinterpret_cast<const uint4*>(qg + ((uq_draft_row(x, sg.b, n / G)) * p.HQ + sg.hk * G + n % G) * D) + a);
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(qg + (uq_draft_row(p, sg.b, j_first + n / G) * p.HQ + sg.hk * G + n % G) * D) + a);
           const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
           for (int j = 0; j < 4; j++) amax = max(amax, max(w4[j] & 0x7FFFu, (w4[j] >> 16) & 0x7FFFu));
@@ -1287,7 +1289,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           const int n = i / (D / 8), a = i % (D / 8);
           uint4 w = make_uint4(0, 0, 0, 0);
           if (n < rows) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(qg + ((uq_draft_row(x, sg.b, n / G)) * p.HQ + sg.hk * G + n % G) * D) + a);
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(qg + (uq_draft_row(p, sg.b, j_first + n / G) * p.HQ + sg.hk * G + n % G) * D) + a);
             w.x = pack_f16x2(__uint_as_float(v.x << 16) * qf, __uint_as_float(v.x & 0xFFFF0000u) * qf);
             w.y = pack_f16x2(__uint_as_float(v.y << 16) * qf, __uint_as_float(v.y & 0xFFFF0000u) * qf);
             w.z = pack_f16x2(__uint_as_float(v.z << 16) * qf, __uint_as_float(v.z & 0xFFFF0000u) * qf);
@@ -1307,7 +1309,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
       // the first segment of an item marks the slots the item does not use as empty
       if (sg.t0 == 0)
         for (int i = st; i < (x.ns_eff - sg.nseg) * rows; i += kSm)
-          p.ml[uq_slot(p, sg.b, sg.hk, sg.nseg + i / rows) * x.BM + i % rows] = -INFINITY;
+          p.ml[uq_slot(p, sg.b, sg.hk, sg.nseg + i / rows) * x.BM + row_off + i % rows] = -INFINITY;
       // (no rendezvous here: the first tile reads none of these before the rendezvous of its reference move)
       UQ_TRACE_SEG(4)
       float l[HW];
@@ -1318,7 +1320,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
       // the common tiles
       int tmask;
       {
-        const int xq = n_glob - Kq - off - (kKeys - 1) - (x.tree_mask ? 1 : 0);
+        const int xq = n_glob - p.K - off - (kKeys - 1) - (x.tree_mask ? 1 : 0);
         tmask = min(n_loc / kKeys, xq < 0 ? 0 : xq / kKeys + 1);
       }
       for (int t = sg.t0; ok && t < sg.t1; t++, cnt++) {
@@ -1387,15 +1389,15 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         const float ck = C::kBS ? csc0 : csc0 * uq_scale_f32(rf & 0xFFu);   // block-scaled scores carry the keys' scales already
         // only a tile that reaches the end of the sequence or the draft positions needs masks (same answer in every thread)
         // (chain: draft token 0 is seen by every row, so the masks start at draft 1; a tree may hide draft 0 from some rows)
-        const bool need_mask = t * kKeys + kKeys - 1 >= n_loc || off + t * kKeys + kKeys - 1 + (x.tree_mask ? 1 : 0) > n_glob - Kq;
+        const bool need_mask = t * kKeys + kKeys - 1 >= n_loc || off + t * kKeys + kKeys - 1 + (x.tree_mask ? 1 : 0) > n_glob - p.K;
         bool live = true;
         uint32_t vmask = 0xFFFFFFFFu;   // bit i: row r0 + i sees this key
         if (need_mask) {
           const int key = t * kKeys + kk;
           live = key < n_loc;
-          const int td = off + key - (n_glob - Kq);   // >= 0: the key is draft token td
+          const int td = off + key - (n_glob - p.K);   // >= 0: the key is draft token td
           if (!live) vmask = 0u;
-          else if (td >= 0) vmask = draft_rows(x.tree_mask, Kq, sg.b, td, r0, HW, rows, G, j_first);
+          else if (td >= 0) vmask = draft_rows(x.tree_mask, p.K, sg.b, td, r0, HW, rows, G, j_first);
         }
         uint8_t* pt = sm + C::oP + (buf / C::kPPer) * C::kPTile + kk * 128;
         const int pc0 = (buf % C::kPPer) * (NT / 8) + r0 / 8;
@@ -1564,8 +1566,8 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
       UQ_TRACE_SEG(8)
       {
         const size_t slot = uq_slot(p, sg.b, sg.hk, sg.slot);
-        float* mo = p.mo + slot * x.BM * D;
-        float* ml = p.ml + slot * x.BM;
+        float* mo = p.mo + (slot * x.BM + row_off) * D;
+        float* ml = p.ml + slot * x.BM + row_off;
         const float* mr = mref + mcur * NT;
         const float osc = pow2_f32((int)wr[4 + mcur] - 127);   // O^T was accumulated relative to the segment's V reference
         bool bad = false;   // an infinity or a NaN in the sums: a probability or a V value overflowed fp16 somewhere in the segment
@@ -1766,7 +1768,7 @@ bool uq_verify_tc_serves(const UQParams& p, const UQLaunch& x) {
 // Partial slots the kernel uses per (sequence, kv head): at most the caller's nsplit, and no more than an item can span.
 // The flat list gives a CTA ceil(total / SMs) tiles and total >= Hkv x (tiles of the longest item), so an item spans at
 // most ceil(SMs / Hkv) + 1 CTAs; slots beyond that would only be marked empty by the kernel and skipped by the combine.
-int uq_verify_tc_splits(const UQParams& p, const UQLaunch&) {
+int uq_verify_tc_splits(const UQParams& p, const UQLaunch& x) {
   static std::atomic<int> cached[64];
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -1775,7 +1777,7 @@ int uq_verify_tc_splits(const UQParams& p, const UQLaunch&) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) { cudaGetLastError(); return p.nsplit; }
     if (dev >= 0 && dev < 64) cached[dev].store(sms, std::memory_order_relaxed);
   }
-  const int span = (sms + p.HKV - 1) / p.HKV + 1;
+  const int span = (sms + p.HKV * x.chunks - 1) / (p.HKV * x.chunks) + 1;
   return std::max(1, std::min(p.nsplit, span));
 }
 

@@ -106,8 +106,7 @@ def test_scale_extremes():
 
 @pytest.mark.parametrize("K,HQ,HKV,D", [(16, 16, 2, 128), (12, 16, 2, 128), (8, 32, 2, 64), (16, 8, 1, 256), (13, 14, 2, 128)])
 def test_more_than_64_query_rows_run_as_draft_chunks_on_the_tensor_core_kernel(K, HQ, HKV, D):
-    """K * group between 65 and 128 rows: consecutive drafts are verified in chunks of at most 64 rows, each chunk against
-    the sequence cut after it; answers follow the oracle, short sequences (fewer tokens than drafts) included."""
+    """K * group between 65 and 128 rows: consecutive drafts are verified in chunks of at most 64 rows; answers follow the oracle, short sequences (fewer tokens than drafts) included."""
     rng = np.random.default_rng(K * 100 + HQ)
     B, PAGE = 3, 32
     sl = np.array([900, 5, 333], np.int32)       # 5 < K: some drafts see nothing or only part of the tokens
@@ -130,6 +129,25 @@ def test_more_than_64_query_rows_run_as_draft_chunks_on_the_tensor_core_kernel(K
     o, lse = uq_cuda.uq_decode_partial(q, *args)
     merged = uq_cuda.uq_merge(o.unsqueeze(0), lse.unsqueeze(0))
     check_close(merged.float().cpu().numpy(), ref, f"K={K} partial")
+
+
+@pytest.mark.parametrize("nsplit", [1, 2, None])
+@pytest.mark.parametrize("K,HQ,HKV,D", [(16, 16, 2, 128), (9, 8, 1, 256), (5, 28, 2, 64)])
+def test_two_chunks_of_drafts_share_one_launch(K, HQ, HKV, D, nsplit):
+    """65..128 query rows: both chunks are work items of one attention launch and one combine (two launches in all), rows that
+    divide unevenly between them, a sequence without keys, and one slot per item (whole items per CTA) included."""
+    rng = np.random.default_rng(K + D)
+    B, PAGE = 5, 16
+    sl = np.array([700, 0, 3, 128, 129], np.int32)
+    npg = -(-int(sl.max()) // PAGE)
+    kc, ks = O.quantize_fp4(rng.standard_normal((B * npg, HKV, PAGE, D)).astype(np.float32))
+    vc, vs = O.quantize_fp4(rng.standard_normal((B * npg, HKV, PAGE, D)).astype(np.float32))
+    bt = rng.permutation(B * npg).astype(np.int32).reshape(B, npg)
+    qb = O.bf16_bits(rng.standard_normal((B, K, HQ, D)).astype(np.float32))
+    n0 = uq_cuda.launch_count()
+    out = uq_cuda.uq_decode_cuda(dev(qb.view(np.int16), torch.bfloat16), *(dev(a) for a in (kc, ks, vc, vs, bt, sl)), nsplit=nsplit)
+    assert uq_cuda.launch_count() == n0 + 2 and uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
+    check_close(out.float().cpu().numpy(), O.reference(qb, kc, ks, vc, vs, bt, sl), f"K={K} nsplit={nsplit}")
 
 
 @pytest.mark.parametrize("PAGE,D,fmt", [(16, 128, 0), (256, 128, 0), (512, 128, 0), (256, 64, 0), (1024, 256, 0), (256, 128, 1), (48, 128, 0),
