@@ -113,9 +113,6 @@ __device__ unsigned long long g_tc_prof[5][8];
 #ifndef UQ_SB128
 #define UQ_SB128 3   // K / S^T / P^T ring depth at head_dim 128
 #endif
-#ifndef UQ_PROD2
-#define UQ_PROD2 1   // copy warps beside the first: 0 one warp issues everything; 1 K side / V side; 2 K codes / V codes / both scale slices
-#endif
 #ifndef UQ_QKMERGE
 #define UQ_QKMERGE 32   // block-scaled Q.K with up to this many rows: the leading and the remainder tile of Q are ONE B operand of 2 NT rows (half the Q.K instructions; the softmax adds the two halves of S^T); 0 = never
 #endif
@@ -230,12 +227,14 @@ UQ_DEV void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint
 }
 // contiguous bulk copy (scale pages)
 UQ_DEV void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t pol) {
-  if (UQ_EVICT_FIRST)
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(pol) : "memory");
-  else
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(pol) : "memory");
 }
+// 16 bytes into shared memory by an ordinary asynchronous copy of this thread, and its arrival on `bar` once all copies the
+// thread has issued so far have landed
+UQ_DEV void cp_async16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+UQ_DEV void cp_async_arrive(uint32_t bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
+UQ_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // shared-memory matrix descriptor, 128-byte swizzle (sm_100 format: version bit 46, layout type 2 at bit 61)
 UQ_DEV uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -694,7 +693,8 @@ struct Walker {
 };
 
 // ---------------------------------------------------------------------------------------------- kernel
-template <int D, int NT, int FMT>
+// kAsync: the scale slices come by per-lane asynchronous copies of a third copy warp (see the copy role)
+template <int D, int NT, int FMT, bool kAsync>
 __global__ void __launch_bounds__(cta_threads(NT), 1)
 uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ CUtensorMap map_kc, const __grid_constant__ CUtensorMap map_vc) {
   using C = Cfg<D, NT, FMT>;
@@ -749,7 +749,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   // ---- set-up: barriers, tile prefix, TMEM
   if (tid == 0) {
     // a raw stage is free again after the four K (or relay) warps and the V warps have read it (block-scaled: and after the Q.K instructions have)
-    for (int s = 0; s < kRawStages; s++) { mbar_init(bar_raw_full(s), UQ_PROD2 + 1); mbar_init(bar_raw_empty(s), 4 + (kNV == 8 && kVB == 2 ? 4 : kNV) + (C::kBS ? 1 : 0)); }
+    for (int s = 0; s < kRawStages; s++) { mbar_init(bar_raw_full(s), kAsync ? 2 + 32 : 2); mbar_init(bar_raw_empty(s), 4 + (kNV == 8 && kVB == 2 ? 4 : kNV) + (C::kBS ? 1 : 0)); }
     // role barriers count one arrival per warp (lane 0, after __syncwarp): 128 separate arrivals per tile and
     // barrier serialise in the shared-memory unit and cost more than the work they order
     for (int i = 0; i < kSB; i++) {
@@ -827,10 +827,12 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   // does this pass run segment `ord`?  (pass 1: the marked ones)
   auto take = [&]() -> bool { ord++; return pass == 0 || (ord < 32 * kRedoWords && ((redo[ord >> 5] >> (ord & 31)) & 1u)); };
 
-  if (warp == kWarpProd || (UQ_PROD2 >= 1 && warp == kWarpProd + 2) || (UQ_PROD2 == 2 && warp == kWarpProd + 3)) {
+  if (warp == kWarpProd || warp == kWarpProd + 2 || (kAsync && warp == kWarpProd + 3)) {
     // ================================================================= producer
-    // what this warp copies of every tile: bit 0 K codes, bit 1 V codes, bit 2 K scales, bit 3 V scales
-    const int side = (UQ_PROD2 == 0 ? 15 : (UQ_PROD2 == 1 ? (warp == kWarpProd ? 5 : 10) : (warp == kWarpProd ? 1 : (warp == kWarpProd + 2 ? 2 : 12)))) & ((UQ_ABL & 2048) ? 3 : 15);
+    // Two warps, K side and V side: a lane per unit, a tensor copy of the codes and a bulk copy of the scale bytes.  A copy costs
+    // its issuing warp 250-350 cycles, one after the other; where that sets the pace (dispatch_rows) a third warp takes both
+    // scale slices by ordinary asynchronous copies, 16 bytes per lane.
+    const int side = warp == kWarpProd ? 5 : (!kAsync || warp == kWarpProd + 2 ? 10 : 0);   // bit 0 K codes, 1 V codes, 2 K scales, 3 V scales; 0: the third warp
     // a copy moves one unit: a whole page of up to 128 tokens, or a 128-token part of a larger page
     const int unit = prm.unit, ppt = kKeys / unit, spp = p.PAGE / unit;   // tokens per unit, units per tile (1 .. 8), units per page
     // (units per page are a power of two for power-of-two pages: shifts and masks then, no division in the per-tile chain)
@@ -861,7 +863,25 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         if (!ok) break;
         const uint32_t dst = sm_a + C::oRaw + stage * C::kRawStage;
         if (lane == 0) { UQ_TRACE(0, cnt) }
-        if (lane == 0) mbar_expect_tx(bar_raw_full(stage), (uint32_t)vp * ((uint32_t)__popc(side & 3) * page_bytes_codes + (uint32_t)__popc(side & 12) * page_bytes_scales));
+        if (kAsync && side == 0) {
+          // a lane copies pieces of 16 bytes (16 / kScaleB keys of one unit) of both slices
+          const int unit_sh = __ffs(unit) - 1;   // (a power of two from 16 to 128)
+          constexpr int kPieces = C::kRawScales / 16;
+#pragma unroll
+          for (int i0 = 0; i0 < kPieces; i0 += 32) {
+            const int i = i0 + lane, key = i * (16 / C::kScaleB), u = key >> unit_sh;
+            const int upid = __shfl_sync(0xffffffffu, pid, u & 31);
+            if (i < kPieces && u < vp) {
+              const int in_page = spp_p2 ? (t * ppt + u) & (spp - 1) : (t * ppt + u) % spp;
+              const size_t row = (size_t)(((long long)upid * p.HKV + sg.hk) * p.PAGE + in_page * unit + (key & (unit - 1)));
+              cp_async16(dst + C::kOffKS + i * 16, p.ks + row * C::kScaleB);
+              cp_async16(dst + C::kOffVS + i * 16, p.vs + row * C::kScaleB);
+            }
+          }
+          cp_async_arrive(bar_raw_full(stage));
+          continue;
+        }
+        if (lane == 0) mbar_expect_tx(bar_raw_full(stage), (uint32_t)vp * (page_bytes_codes + (kAsync ? 0u : page_bytes_scales)));
         __syncwarp();
         if (lane < vp) {
           // first cache row of this unit of (page, head); 64-bit: a cache may hold more than 2^31 / PAGE (page, head) slices
@@ -871,11 +891,12 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           // block-scaled: the K map unpacks (a page lands as PAGE x 128 bytes); the bytes counted on the barrier are the packed ones
           if (side & 1) tma_load_2d(dst + lane * (C::kBS ? 2 : 1) * page_bytes_codes, &map_kc, 0, (int)row0, fb, l2pol);
           if (side & 2) tma_load_2d(dst + C::kOffVC + lane * page_bytes_codes, &map_vc, 0, (int)row0, fb, l2pol);
-          if (side & 4) bulk_load(dst + C::kOffKS + lane * page_bytes_scales, p.ks + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
-          if (side & 8) bulk_load(dst + C::kOffVS + lane * page_bytes_scales, p.vs + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
+          if (!kAsync && (side & 4)) bulk_load(dst + C::kOffKS + lane * page_bytes_scales, p.ks + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
+          if (!kAsync && (side & 8)) bulk_load(dst + C::kOffVS + lane * page_bytes_scales, p.vs + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
         }
       }
     }
+    if (kAsync && side == 0) cp_async_wait_all();   // (none of its copies outlives the role)
     if (!ok) {
       // Giving up (a wait ran out somewhere in the CTA): copies this warp requested may still be in flight towards this CTA's
       // shared memory, which must not be left while they are.  Wait for the full barrier of every stage it armed, for about
@@ -1695,10 +1716,17 @@ bool cached_map(CUtensorMap* out, const MapKey& key) {
   return true;
 }
 
-template <int D, int NT, int FMT>
+// a copy moves gcd(PAGE, 128) tokens: a page of up to 128 tokens, a 128-token part of a larger one, or their common part
+int copy_unit(const UQParams& p) {
+  int u = kKeys;
+  while (p.PAGE % u) u >>= 1;
+  return u;
+}
+
+template <int D, int NT, int FMT, bool kAsync>
 cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   using C = Cfg<D, NT, FMT>;
-  auto kern = uq_verify_tc_kernel<D, NT, FMT>;
+  auto kern = uq_verify_tc_kernel<D, NT, FMT, kAsync>;
   static std::atomic<bool> ready[64];
   static std::atomic<int> sm_counts[64];
   int dev = 0;
@@ -1719,8 +1747,7 @@ cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   const long long max_tiles = ((long long)p.max_pages * p.PAGE + kKeys - 1) / kKeys;
   prm.chunk_min = x.ns_eff >= 2 ? (int)((max_tiles + x.ns_eff - 2) / (x.ns_eff - 1)) : 1;
   CUtensorMap mk, mv;
-  int box_rows = kKeys;   // a copy moves gcd(PAGE, 128) tokens: a page of up to 128 tokens, a 128-token part of a larger one, or their common part
-  while (p.PAGE % box_rows) box_rows >>= 1;
+  const int box_rows = copy_unit(p);
   prm.unit = box_rows;
   if (!cached_map(&mk, MapKey{p.kc, C::kCodeRow, box_rows, C::kBS ? 1 : 0}) || !cached_map(&mv, MapKey{p.vc, C::kCodeRow, box_rows, 0})) return cudaErrorInvalidValue;
   const int sms = sm_counts[dev].load(std::memory_order_relaxed);
@@ -1783,9 +1810,16 @@ int uq_verify_tc_splits(const UQParams& p, const UQLaunch& x) {
 
 template <int D, int FMT>
 static cudaError_t dispatch_rows(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
-  if (x.rows <= 16) return tc::launch<D, 16, FMT>(p, x, s);
-  if (x.rows <= 32) return tc::launch<D, 32, FMT>(p, x, s);
-  return tc::launch<D, 64, FMT>(p, x, s);
+  // Small units mean many copies per tile, and their issue becomes the kernel's pace: the scale slices then come by a third copy
+  // warp.  GPU time without / with it (B=8, 8 K tokens; 16 sequences of 1 K .. 4 K for the one marked *): head_dim 128, 16-token pages
+  // 51.6 / 46.6 us at 64 rows, 40.9 / 34.3 at 16, NVFP4 52.9 / 45.1; 32-token pages 34.2 / 32.0 at 16 rows, but 45.4 / 46.7 at 64, where
+  // issue slots are short; 64-token pages level; head_dim 64, whose tiles are half the bytes: 16-token pages * 32.4 / 28.2, 32-token
+  // 35.8 / 32.8, 64-token 32.8 / 32.1.
+  const int unit = tc::copy_unit(p);
+  const bool some = unit <= 32 || D == 64, few = unit == 16;
+  if (x.rows <= 16) return some ? tc::launch<D, 16, FMT, true>(p, x, s) : tc::launch<D, 16, FMT, false>(p, x, s);
+  if (x.rows <= 32) return some ? tc::launch<D, 32, FMT, true>(p, x, s) : tc::launch<D, 32, FMT, false>(p, x, s);
+  return few ? tc::launch<D, 64, FMT, true>(p, x, s) : tc::launch<D, 64, FMT, false>(p, x, s);
 }
 
 cudaError_t uq_verify_tc_dispatch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {

@@ -150,6 +150,31 @@ def test_two_chunks_of_drafts_share_one_launch(K, HQ, HKV, D, nsplit):
     check_close(out.float().cpu().numpy(), O.reference(qb, kc, ks, vc, vs, bt, sl), f"K={K} nsplit={nsplit}")
 
 
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("D,PAGE", [(64, 16), (64, 48), (64, 128), (128, 16), (128, 32), (256, 16), (256, 32)])
+@pytest.mark.parametrize("rows", [8, 32, 64])
+def test_scale_slices_of_small_copies_come_by_a_third_warp(D, PAGE, rows, fmt):
+    """Small copy units: the scale bytes arrive 16 bytes per lane (1 .. 8 keys each, up to four pieces per lane), units past a
+    sequence's end are left out; lengths that end inside a unit, on its edge and one key past a tile."""
+    rng = np.random.default_rng(D + PAGE + rows)
+    B, HKV, G = 4, 2, 8
+    K = rows // G
+    sl = np.array([1, 128 + PAGE, 129, 5 * 128 - 3], np.int32)
+    npg = -(-int(sl.max()) // PAGE)
+    shape = lambda row: (B * npg, HKV, PAGE, row)
+    kc, vc = (rng.integers(0, 256, shape(D // 2), dtype=np.uint8) for _ in range(2))
+    lo, hi, per = (125, 130, 32) if fmt == 0 else (0x30, 0x40, 16)
+    ks, vs = (rng.integers(lo, hi, shape(D // per)).astype(np.uint8) for _ in range(2))
+    bt = rng.permutation(B * npg).astype(np.int32).reshape(B, npg)
+    qb = O.bf16_bits(0.3 * rng.standard_normal((B, K, HKV * G, D)).astype(np.float32))
+    ref = O.reference(qb, kc, ks, vc, vs, bt, sl) if fmt == 0 else O.reference_nvfp4(qb, kc, ks, vc, vs, bt, sl, 0.5, 0.5)
+    out = uq_cuda.uq_decode_cuda(dev(qb.view(np.int16), torch.bfloat16), *(dev(a) for a in (kc, ks, vc, vs, bt, sl)),
+                                 **(dict(fmt=1, k_ts=0.5, v_ts=0.5) if fmt else {}))
+    assert uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
+    check_close(out.float().cpu().numpy(), ref, f"PAGE={PAGE}")
+
+
 @pytest.mark.parametrize("PAGE,D,fmt", [(16, 128, 0), (256, 128, 0), (512, 128, 0), (256, 64, 0), (1024, 256, 0), (256, 128, 1), (48, 128, 0),
                                          (96, 128, 0), (80, 64, 0), (192, 256, 0), (48, 128, 1), (144, 128, 0), (24, 128, 0), (40, 64, 0)])
 def test_page_sizes_from_16_to_1024_tokens(PAGE, D, fmt):
