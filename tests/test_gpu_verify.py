@@ -172,7 +172,10 @@ def test_scale_slices_of_small_copies_come_by_a_third_warp(D, PAGE, rows, fmt):
     out = uq_cuda.uq_decode_cuda(dev(qb.view(np.int16), torch.bfloat16), *(dev(a) for a in (kc, ks, vc, vs, bt, sl)),
                                  **(dict(fmt=1, k_ts=0.5, v_ts=0.5) if fmt else {}))
     assert uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
-    check_close(out.float().cpu().numpy(), ref, f"PAGE={PAGE}")
+    # (a sequence of one key returns that key's value, up to 24 here, rounded to bf16 - half an ulp is 2^-9 of it - while the rule's mean
+    # bound is absolute and meant for outputs of O(1): compared relative to the largest)
+    mx = np.abs(ref).max()
+    check_close(out.float().cpu().numpy() / mx, ref / mx, f"PAGE={PAGE}")
 
 
 @pytest.mark.parametrize("PAGE,D,fmt", [(16, 128, 0), (256, 128, 0), (512, 128, 0), (256, 64, 0), (1024, 256, 0), (256, 128, 1), (48, 128, 0),
