@@ -171,6 +171,9 @@ cudaError_t run_one(const UQParams& p, UQLaunch x, float* o_part, float* lse_par
   cudaError_t e;
   const bool timed = t_ev_before && t_ev_after;
   if (timed) cudaEventRecord(t_ev_before, s);
+  // (UQ_B200_CFG="pdl=0" turns programmatic dependent launches off; an event between two launches needs them apart)
+  static const bool pdl_on = !(std::getenv("UQ_B200_CFG") && std::strstr(std::getenv("UQ_B200_CFG"), "pdl=0"));
+  x.pdl = tc && pdl_on && !timed;
   if (tc) {
     x.ns_eff = uq_verify_tc_splits(p, x);
     e = uq_verify_tc_dispatch(p, x, s);
@@ -185,10 +188,7 @@ cudaError_t run_one(const UQParams& p, UQLaunch x, float* o_part, float* lse_par
   if (timed) cudaEventRecord(t_ev_after, s);
   if (e != cudaSuccess) return e;
   g_launches += 2;
-  // (after the tcgen05 kernel, which signals its dependents at once, the combine is launched as a programmatic dependent;
-  // UQ_B200_CFG="pdl=0" turns that off)
-  static const bool pdl_on = !(std::getenv("UQ_B200_CFG") && std::strstr(std::getenv("UQ_B200_CFG"), "pdl=0"));
-  return uq_combine_dispatch(p, x, o_part, lse_part, push, tc && pdl_on && !timed, s);
+  return uq_combine_dispatch(p, x, o_part, lse_part, push, x.pdl != 0, s);
 }
 
 }  // namespace

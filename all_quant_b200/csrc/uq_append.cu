@@ -134,6 +134,8 @@ __global__ void __launch_bounds__(128) uq_append_kernel(uint8_t* __restrict__ kc
                                                         uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                         const int64_t* __restrict__ slots, int T_tok, int HKV, int D, int PAGE, int nstream,
                                                         int flags, float c) {
+  uq_pdl_release();
+  uq_pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int total = T_tok * HKV * nstream;
@@ -348,6 +350,8 @@ __global__ void __launch_bounds__(256) uq_append_bulk_kernel(uint8_t* __restrict
                                                              uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                              const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
                                                              int PAGE, int page_shift, int paper, float c) {
+  uq_pdl_release();
+  uq_pdl_wait();
   constexpr bool kExactTies = sizeof(T) == 4;   // fp32 inputs can sit anywhere: half-way values are corrected by comparison
   constexpr int NP = bulk_pieces<T>();          // pieces per thread: 128 bytes of input in flight
   const int stream = blockIdx.y;
@@ -466,9 +470,9 @@ bool bulk_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const T* ke
   const unsigned per_block = (UQ_BULK_THREADS / 32u) * 32u * bulk_pieces<T>();
   const dim3 grid((unsigned)((np + per_block - 1) / per_block), (unsigned)nstream);
   if (flags & kRotateK)
-    uq_append_bulk_kernel<T, true><<<grid, UQ_BULK_THREADS, 0, s>>>(kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c);
+    uq_launch(uq_append_bulk_kernel<T, true>, grid, UQ_BULK_THREADS, 0, s, true, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c);
   else
-    uq_append_bulk_kernel<T, false><<<grid, UQ_BULK_THREADS, 0, s>>>(kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c);
+    uq_launch(uq_append_bulk_kernel<T, false>, grid, UQ_BULK_THREADS, 0, s, true, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c);
   return true;
 }
 
@@ -481,6 +485,8 @@ __global__ void __launch_bounds__(128) uq_append_nvfp4_kernel(uint8_t* __restric
                                                               uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                               const int64_t* __restrict__ slots, int T_tok, int HKV, int D, int PAGE, float k_ts,
                                                               float v_ts) {
+  uq_pdl_release();
+  uq_pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= T_tok * HKV * 2) return;
@@ -563,6 +569,8 @@ __global__ void __launch_bounds__(256) uq_append_nvfp4_bulk_kernel(uint8_t* __re
                                                                    uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                                    const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
                                                                    int PAGE, int page_shift, float k_ts, float v_ts) {
+  uq_pdl_release();
+  uq_pdl_wait();
   constexpr int NP = bulk_pieces<T>();
   constexpr bool kAddZero = sizeof(T) == 4;   // fp32 inputs: any product can underflow, +0 is added after the multiplication
   // a 16-bit input's smallest non-zero magnitude (2^-133 bf16, 2^-24 fp16) times the reciprocal stays a normal number
@@ -672,13 +680,15 @@ bool bulk_nvfp4_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const
   if ((PAGE & (PAGE - 1)) == 0) { shift = 0; while ((1 << shift) < PAGE) shift++; }
   const unsigned per_block = (UQ_BULK_THREADS / 32u) * 32u * bulk_pieces<T>();
   const dim3 grid((unsigned)((np + per_block - 1) / per_block), 2u);
-  uq_append_nvfp4_bulk_kernel<T><<<grid, UQ_BULK_THREADS, 0, s>>>(kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, k_ts, v_ts);
+  uq_launch(uq_append_nvfp4_bulk_kernel<T>, grid, UQ_BULK_THREADS, 0, s, true, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, k_ts, v_ts);
   return true;
 }
 
 // The transform alone (the queries of a cache whose keys were rotated): one warp per row, out may be x.
 template <typename T>
 __global__ void __launch_bounds__(128) uq_fwht_kernel(const T* __restrict__ x, T* __restrict__ out, long long rows, int D) {
+  uq_pdl_release();
+  uq_pdl_wait();
   const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -707,9 +717,9 @@ cudaError_t uq_fwht_dispatch(const void* x, void* out, long long rows, int D, in
   const long long blocks = (rows + 3) / 4;
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
   switch (dtype) {
-    case 0: uq_fwht_kernel<float><<<(int)blocks, 128, 0, s>>>((const float*)x, (float*)out, rows, D); break;
-    case 1: uq_fwht_kernel<__nv_bfloat16><<<(int)blocks, 128, 0, s>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, D); break;
-    default: uq_fwht_kernel<__half><<<(int)blocks, 128, 0, s>>>((const __half*)x, (__half*)out, rows, D); break;
+    case 0: uq_launch(uq_fwht_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, true, (const float*)x, (float*)out, rows, D); break;
+    case 1: uq_launch(uq_fwht_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, true, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, D); break;
+    default: uq_launch(uq_fwht_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, true, (const __half*)x, (__half*)out, rows, D); break;
   }
   return cudaGetLastError();
 }
@@ -734,9 +744,9 @@ cudaError_t uq_append_nvfp4_dispatch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint
   }
   const int blocks = (int)((warps + 3) / 4);
   switch (dtype) {
-    case 0: uq_append_nvfp4_kernel<float><<<blocks, 128, 0, s>>>(kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
-    case 1: uq_append_nvfp4_kernel<__nv_bfloat16><<<blocks, 128, 0, s>>>(kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
-    default: uq_append_nvfp4_kernel<__half><<<blocks, 128, 0, s>>>(kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
+    case 0: uq_launch(uq_append_nvfp4_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
+    case 1: uq_launch(uq_append_nvfp4_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
+    default: uq_launch(uq_append_nvfp4_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
   }
   return cudaGetLastError();
 }
@@ -769,9 +779,9 @@ cudaError_t uq_append_dispatch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* v
   }
   const int blocks = (int)((warps + 3) / 4);
   switch (dtype) {
-    case 0: uq_append_kernel<float><<<blocks, 128, 0, s>>>(kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
-    case 1: uq_append_kernel<__nv_bfloat16><<<blocks, 128, 0, s>>>(kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
-    default: uq_append_kernel<__half><<<blocks, 128, 0, s>>>(kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
+    case 0: uq_launch(uq_append_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
+    case 1: uq_launch(uq_append_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
+    default: uq_launch(uq_append_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
   }
   return cudaGetLastError();
 }

@@ -9,6 +9,11 @@
 
 namespace {
 
+// The kernel after a combine of up to this many blocks is set up from its start on (the next layer's append or verify call: 0.3 to
+// 1 us less per call); a larger grid takes more than one wave of blocks and lets go at its end (32 sequences, 4096 blocks: 446 us a
+// call, 454 when released at the start).
+constexpr unsigned kReleaseBlocks = 2048;
+
 // Partials of (b, hk) live in scratch slots s = 0..ns_eff-1, rows r = j*G + g with stride BM.
 // kOut: 0 bf16 result, 1 fp32 partial + lse2 to the caller's arrays, 2 the same partial to every rank's exchange buffer
 template <int kOut>
@@ -17,10 +22,9 @@ __global__ void __launch_bounds__(128) uq_combine_kernel(const UQParams p, const
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);   // over [B, K, HQ]
   const int lane = threadIdx.x & 31;
   const int total = p.B * p.K * p.HQ;
-  // Launched as a programmatic dependent of the attention kernel (its blocks may become resident while that kernel's last
-  // CTAs still run): nothing of the partials is read before the whole attention grid has completed and its writes are visible.
-  // (A no-op when the launch carries no such dependency.)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (nothing of the partials is read before the whole attention grid has completed and its writes are visible)
+  if (gridDim.x <= kReleaseBlocks) uq_pdl_release();
+  uq_pdl_wait();
   if (row < total) {
   const int h = row % p.HQ, j = (row / p.HQ) % p.K, b = row / (p.HQ * p.K);
   const int hk = h / x.G, r = j * x.G + (h % x.G);
@@ -198,22 +202,11 @@ cudaError_t uq_combine_dispatch(const UQParams& p, const UQLaunch& x, float* o_p
   const int rows = p.B * p.K * p.HQ;
   if (rows == 0) return cudaSuccess;
   const UQPeerPush none{};
-  // programmatic stream serialisation: the launch may be set up while the attention kernel before it on the stream is still
-  // running (that kernel signals early); the combine's first instruction waits for that kernel's completion
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((rows + 3) / 4);
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  const dim3 grid((rows + 3) / 4);
   float* no_f = nullptr;
-  if (push) return cudaLaunchKernelEx(&cfg, uq_combine_kernel<2>, p, x, no_f, no_f, *push);
-  if (o_part) return cudaLaunchKernelEx(&cfg, uq_combine_kernel<1>, p, x, o_part, lse_part, none);
-  return cudaLaunchKernelEx(&cfg, uq_combine_kernel<0>, p, x, no_f, no_f, none);
+  if (push) return uq_launch(uq_combine_kernel<2>, grid, 128u, 0, s, pdl, p, x, no_f, no_f, *push);
+  if (o_part) return uq_launch(uq_combine_kernel<1>, grid, 128u, 0, s, pdl, p, x, o_part, lse_part, none);
+  return uq_launch(uq_combine_kernel<0>, grid, 128u, 0, s, pdl, p, x, no_f, no_f, none);
 }
 
 cudaError_t uq_merge_dispatch(const float* o, const float* lse, int R, size_t rows, int D, void* out, cudaStream_t s) {

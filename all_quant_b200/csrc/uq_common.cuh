@@ -10,6 +10,30 @@
 
 #define UQ_DEV __device__ __forceinline__
 
+// ---- programmatic dependent launch ------------------------------------------------------------------
+// Every kernel of a call's chain (append, rotate, verify, combine) is launched as a programmatic dependent of what precedes it
+// on the stream: its blocks may be set up while that kernel's last blocks still run.  uq_pdl_wait() returns once everything
+// before it on the stream has completed with its writes visible; every block of every such kernel executes it (a grid whose
+// blocks left without it could complete before its predecessor, and the kernel after it would start too early), and none
+// touches global memory before it.  uq_pdl_release() lets the next kernel be set up as soon as all blocks of this one have
+// started.  Both are no-ops in an ordinary launch.
+UQ_DEV void uq_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+UQ_DEV void uq_pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t uq_launch(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, bool dependent, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = dependent ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // ---- what the host adds to UQParams for one launch -------------------------------------------------
 struct UQLaunch {
   const int32_t* pos_offset;  // [B] global position of shard-local key 0 (nullptr = 0)
@@ -24,6 +48,7 @@ struct UQLaunch {
   // are cut into `chunks` runs of `per` consecutive drafts, each a work item of its own on the whole sequence, with rows
   // chunk * per * G .. of the partial slots.  One chunk of K drafts otherwise.
   int chunks, per;
+  int pdl;                    // launch the kernels as programmatic dependents of what precedes them on the stream
   unsigned int* status;       // this device's status record (4 words), see uq_report
   int expire_id;              // 0, or (for the test of the give-up path) 30: the softmax role never announces the query tile of a
                               // segment, so the wait on barrier 30 runs out after its full limit on an otherwise healthy kernel

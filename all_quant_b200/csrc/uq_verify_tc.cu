@@ -702,13 +702,12 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   // compiler keeps every access in the shared state space (ld.shared / st.shared instead of generic loads and stores)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   UQ_TRACE_CTA_T(0)
-  // the combine kernel that follows on the stream may be set up now (its blocks wait for this grid's completion themselves)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const UQParams& p = prm.p;
   const UQLaunch& x = prm.x;
   uint8_t* sm = smem_raw;
   const uint32_t sm_a = smem_u32(sm);
   if (sm_a & 1023u) {   // never expected; the swizzled layouts below would be wrong
+    uq_pdl_wait();
     if (threadIdx.x == 0) uq_report(prm.x.status, 2u, sm_a, 0u);
     return;
   }
@@ -765,6 +764,11 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   }
   uint32_t* redo = reinterpret_cast<uint32_t*>(sm + C::oRedo);
   for (int i = tid; i <= kRedoWords; i += kThreads) redo[i] = 0u;
+  if (warp == kWarpMma) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sm_a + C::oTmemSlot) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  uq_pdl_wait();   // from here on global memory is read and written
   {
     // the queries (B x K x Hq x D bf16, read once per segment by whichever CTA gets it) go to L2 now, a slice per CTA, while
     // the set-up below runs: the first segment's conversion and every later one then find them there
@@ -790,10 +794,6 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
     Walker w0;
     w0.init(prefix, p.B, p.HKV, x.chunks, x.ns_eff, prm.chunk_min, seg_weight(NT));
     w0.list(seglist, lane);
-  }
-  if (warp == kWarpMma) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sm_a + C::oTmemSlot) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -1637,6 +1637,9 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   UQ_TRACE_CTA_T(4)
   UQ_TRACE_CTA_V(5, cnt)
   UQ_TRACE_CTA_V(6, seg_i)
+  // Not before here: released at its start, the combine's blocks crowd onto the first SMs that fall free (one sequence of 131 K
+  // tokens at head_dim 256: 86.5 us a call, 78.9 with the release at the end of the CTA).
+  uq_pdl_release();
   // ---- common exit: TMEM goes back before the CTA ends
   if (warp == kWarpMma) {
     tc_fence_after();
@@ -1752,8 +1755,7 @@ cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   if (!cached_map(&mk, MapKey{p.kc, C::kCodeRow, box_rows, C::kBS ? 1 : 0}) || !cached_map(&mv, MapKey{p.vc, C::kCodeRow, box_rows, 0})) return cudaErrorInvalidValue;
   const int sms = sm_counts[dev].load(std::memory_order_relaxed);
   if (sms <= 0) return cudaErrorInitializationError;
-  kern<<<sms, cta_threads(NT), C::kSmem, s>>>(prm, mk, mv);
-  return cudaGetLastError();
+  return uq_launch(kern, dim3(sms), cta_threads(NT), C::kSmem, s, x.pdl != 0, prm, mk, mv);
 }
 
 }  // namespace tc

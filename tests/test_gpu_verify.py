@@ -345,3 +345,41 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_call_is_unaffected(monkey
         out = uq_cuda.uq_decode_cuda(q, *args)
         assert uq_cuda.last_status() == (0, 0, 0, 0) and uq_cuda.last_path() == 2
         check_close(out.float().cpu().numpy(), c.ref, "call after a wait that ran out")
+
+@pytest.mark.parametrize("rotate", [False, True])
+def test_a_chain_of_calls_needs_no_synchronisation(rotate):
+    """Every kernel is set up while the one before it on the stream still runs and waits for it before it touches memory: steps
+    that write the cache, the queries and the scratch the neighbouring steps read give the bits of the same steps run apart."""
+    B, K, HQ, HKV, D, PAGE, ctx, steps = 4, 2, 16, 4, 128, 64, 900, 12
+    g = torch.Generator(device="cuda").manual_seed(5)
+    npg = -(-ctx // PAGE)
+    bt = torch.randperm(B * npg, generator=g, device="cuda").to(torch.int32).view(B, npg)
+    key = torch.randn(B * ctx, HKV, D, generator=g, device="cuda").bfloat16()
+    value = torch.randn(B * ctx, HKV, D, generator=g, device="cuda").bfloat16()
+    pos = torch.arange(ctx, device="cuda").repeat(B)
+    slots = bt.long().repeat_interleave(ctx, 0)[torch.arange(B * ctx, device="cuda"), pos // PAGE] * PAGE + pos % PAGE
+    q0 = torch.randn(steps, B, K, HQ, D, generator=g, device="cuda").bfloat16()
+    ws = torch.empty(uq_cuda.workspace_floats(B, K, HQ, HKV, D, 8), device="cuda")
+
+    def run(sync):
+        kc = torch.zeros(B * npg, HKV, PAGE, D // 2, dtype=torch.uint8, device="cuda")
+        ks = torch.zeros(B * npg, HKV, PAGE, D // 32, dtype=torch.uint8, device="cuda")
+        vc, vs = torch.zeros_like(kc), torch.zeros_like(ks)
+        q, out, outs = torch.empty_like(q0[0]), torch.empty_like(q0[0]), []
+        uq_cuda.append_kv(kc, ks, vc, vs, key, value, slots, rotate_k=rotate)
+        for s in range(steps):
+            new = torch.arange(s, B * ctx, steps, device="cuda")   # other tokens in every step, overwritten with a shifted input
+            q.copy_(q0[s])
+            for call in (lambda: uq_cuda.append_kv(kc, ks, vc, vs, key[(new + s + 1) % (B * ctx)], value[new], slots[new], rotate_k=rotate),
+                         lambda: q.copy_(uq_cuda.fwht(q)),
+                         lambda: uq_cuda.uq_decode_cuda(q, kc, ks, vc, vs, bt, torch.full((B,), ctx, dtype=torch.int32, device="cuda"), nsplit=8, workspace=ws, out=out),
+                         lambda: outs.append(out.clone())):
+                call()
+                if sync:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return torch.stack(outs), kc, vs
+
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
+    assert uq_cuda.last_status() == (0, 0, 0, 0)
