@@ -523,7 +523,8 @@ struct Cfg {
   static constexpr int kMaxB = 1024;
   static constexpr int oRedo = oPrefix + (kMaxB + 1) * 4;   // kRedoWords words of per-segment "run again" bits, then one word "any bit set"
   static constexpr int oSegs = oRedo + (kRedoWords + 1) * 4;   // the CTA's first kSegCap segments (SegList), listed once at set-up
-  static constexpr int kSmem = oSegs + (int)sizeof(SegList);
+  static constexpr int oChunk = oSegs + (int)sizeof(SegList);   // what pick_chunk found
+  static constexpr int kSmem = oChunk + 16;
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
   // TMEM columns
   static constexpr int kKCols = kBS ? 4 : D / 2;         // fp16 A operand of S^T: two channels per 32-bit column; block-scaled: the keys' scale bytes
@@ -582,6 +583,33 @@ UQ_DEV int small_quotient(int n, int d) {
   if (r < 0) q--;
   else if (r >= d) q++;
   return q;
+}
+
+// The smallest chunk found that cuts no item into more pieces than it has partial slots (ns >= 2); by one warp.  An item of n
+// tiles spans at most ceil((n - 1) / c) + 1 chunks of c units, so c = `safe`, from the longest sequence, always holds.  Between the CTAs'
+// equal share of the list and `safe` it depends on where the long items happen to lie: lane i tries the i-th of 32 candidates
+// (only an item of more than (ns - 1) * c tiles can break one).  With the bound from the page table's width alone, 32 sequences
+// of 4 K .. 64 K tokens with two slots per item left 28 of the 148 CTAs without work: 446 us a call, 420 with the candidates.
+__device__ __noinline__ int pick_chunk(const int* prefix, int B, int items, int ns, int seg_w) {
+  const int lane = threadIdx.x & 31;
+  int longest = 0;
+  for (int b = lane; b < B; b += 32) longest = max(longest, prefix[b + 1] - prefix[b] - seg_w);
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  const int share = max((items * prefix[B] + (int)gridDim.x - 1) / (int)gridDim.x, 1);
+  const int safe = (longest + ns - 3) / (ns - 1);   // ceil((longest - 1) / (ns - 1))
+  if (share >= safe) return share;
+  const int c = share + (int)((long long)(safe - share) * lane / 32);
+  bool holds = true;
+  for (int b = 0; b < B; b++) {
+    const int wide = prefix[b + 1] - prefix[b], n = wide - seg_w;
+    if (n <= (ns - 1) * c) continue;
+    for (int i = 0; i < items && holds; i++) {
+      const int first = items * prefix[b] + i * wide + seg_w;
+      holds = (first + n - 1) / c - first / c < ns;
+    }
+  }
+  const unsigned good = __ballot_sync(0xffffffffu, holds);
+  return good ? __shfl_sync(0xffffffffu, c, __ffs(good) - 1) : safe;
 }
 
 struct Walker {
@@ -694,7 +722,8 @@ struct Walker {
 
 // ---------------------------------------------------------------------------------------------- kernel
 // kAsync: the scale slices come by per-lane asynchronous copies of a third copy warp (see the copy role)
-template <int D, int NT, int FMT, bool kAsync>
+// kPick: a chunk below the launch's chunk_min is looked for (pick_chunk)
+template <int D, int NT, int FMT, bool kAsync, bool kPick>
 __global__ void __launch_bounds__(cta_threads(NT), 1)
 uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ CUtensorMap map_kc, const __grid_constant__ CUtensorMap map_vc) {
   using C = Cfg<D, NT, FMT>;
@@ -763,6 +792,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
     fence_barrier_init();
   }
   uint32_t* redo = reinterpret_cast<uint32_t*>(sm + C::oRedo);
+  int* chunk_s = reinterpret_cast<int*>(sm + C::oChunk);
   for (int i = tid; i <= kRedoWords; i += kThreads) redo[i] = 0u;
   if (warp == kWarpMma) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sm_a + C::oTmemSlot) : "memory");
@@ -792,7 +822,12 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   if (warp == 0) {   // the CTA's segments, once, for every role (the walker's struct lives in registers here)
     __syncwarp();
     Walker w0;
-    w0.init(prefix, p.B, p.HKV, x.chunks, x.ns_eff, prm.chunk_min, seg_weight(NT));
+    int chunk_min = prm.chunk_min;
+    if constexpr (kPick) {
+      if (p.HKV * x.chunks * prefix[p.B] < (int)gridDim.x * chunk_min) chunk_min = pick_chunk(prefix, p.B, p.HKV * x.chunks, x.ns_eff, seg_weight(NT));
+      if (lane == 0) *chunk_s = chunk_min;
+    }
+    w0.init(prefix, p.B, p.HKV, x.chunks, x.ns_eff, chunk_min, seg_weight(NT));
     w0.list(seglist, lane);
   }
   tc_fence_before();
@@ -821,7 +856,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   auto next_seg = [&](Seg& s) -> bool {
     if (seg_at < seglist->n) { s = seglist->seg[seg_at++]; return true; }
     if (!seglist->more) return false;
-    return wk.next_after(s, seglist, walking, prefix, p.B, p.HKV, x.chunks, x.ns_eff, prm.chunk_min, seg_weight(NT));
+    return wk.next_after(s, seglist, walking, prefix, p.B, p.HKV, x.chunks, x.ns_eff, kPick ? *chunk_s : prm.chunk_min, seg_weight(NT));
   };
   int ord = -1;                    // ordinal of the segment in the CTA's list
   // does this pass run segment `ord`?  (pass 1: the marked ones)
@@ -1726,10 +1761,16 @@ int copy_unit(const UQParams& p) {
   return u;
 }
 
-template <int D, int NT, int FMT, bool kAsync>
-cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
+// an item of n tiles cut into chunks of c tiles spans at most ceil(n / c) + 1 CTAs: this keeps that within ns_eff whatever the lengths
+int chunk_bound(const UQParams& p, const UQLaunch& x) {
+  const long long max_tiles = ((long long)p.max_pages * p.PAGE + kKeys - 1) / kKeys;
+  return x.ns_eff >= 2 ? (int)((max_tiles + x.ns_eff - 2) / (x.ns_eff - 1)) : 1;
+}
+
+template <int D, int NT, int FMT, bool kAsync, bool kPick>
+cudaError_t launch_as(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   using C = Cfg<D, NT, FMT>;
-  auto kern = uq_verify_tc_kernel<D, NT, FMT, kAsync>;
+  auto kern = uq_verify_tc_kernel<D, NT, FMT, kAsync, kPick>;
   static std::atomic<bool> ready[64];
   static std::atomic<int> sm_counts[64];
   int dev = 0;
@@ -1746,9 +1787,7 @@ cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   Params prm;
   prm.p = p;
   prm.x = x;
-  // an item of n tiles cut into chunks of c tiles spans at most ceil(n / c) + 1 CTAs: keep that within ns_eff
-  const long long max_tiles = ((long long)p.max_pages * p.PAGE + kKeys - 1) / kKeys;
-  prm.chunk_min = x.ns_eff >= 2 ? (int)((max_tiles + x.ns_eff - 2) / (x.ns_eff - 1)) : 1;
+  prm.chunk_min = chunk_bound(p, x);
   CUtensorMap mk, mv;
   const int box_rows = copy_unit(p);
   prm.unit = box_rows;
@@ -1756,6 +1795,18 @@ cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   const int sms = sm_counts[dev].load(std::memory_order_relaxed);
   if (sms <= 0) return cudaErrorInitializationError;
   return uq_launch(kern, dim3(sms), cta_threads(NT), C::kSmem, s, x.pdl != 0, prm, mk, mv);
+}
+
+// The equal share of 148 CTAs is at most items x (longest table) / 148 tiles.  Where the bound is above a third of that - two or
+// three slots per item, with the default slot count from 150 items on - it is likely to bind for sequences of different length, and
+// the kernel looks for a smaller chunk (below eight tiles there is nothing to gain).  Elsewhere the code for that stays out: in every launch it cost up to 4 % of calls that
+// never use it (K=1, 8 sequences of 32 K tokens: 83.0 us, 85.8 with it).
+template <int D, int NT, int FMT, bool kAsync>
+cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
+  const long long max_tiles = ((long long)p.max_pages * p.PAGE + kKeys - 1) / kKeys;
+  const int bound = chunk_bound(p, x);
+  const bool pick = x.ns_eff >= 2 && bound >= 8 && 3ll * 148 * bound > (long long)p.B * p.HKV * x.chunks * max_tiles;
+  return pick ? launch_as<D, NT, FMT, kAsync, true>(p, x, s) : launch_as<D, NT, FMT, kAsync, false>(p, x, s);
 }
 
 }  // namespace tc

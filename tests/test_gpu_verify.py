@@ -383,3 +383,30 @@ def test_a_chain_of_calls_needs_no_synchronisation(rotate):
     for a, b in zip(run(False), run(True)):
         assert torch.equal(a, b)
     assert uq_cuda.last_status() == (0, 0, 0, 0)
+
+@pytest.mark.parametrize("nsplit", [2, 3])
+@pytest.mark.parametrize("B,HKV,long_ones,longest,width", [(40, 4, 3, 3000, 3000), (40, 4, 3, 3000, 40000), (150, 1, 1, 9000, 9000), (33, 8, 33, 1500, 1500), (3, 1, 3, 20000, 20000)])
+def test_items_cut_into_no_more_pieces_than_they_have_slots(B, HKV, long_ones, longest, width, nsplit):
+    """Few partial slots and lengths far apart: the CTAs' equal share would cut the long items into more pieces than there are
+    slots, so a larger chunk is chosen (the smallest of a row of candidates that fits, or the one that always does).  The
+    scratch is exactly nsplit slots; a guard behind it stays untouched.  `width`: a page table far wider than the sequences."""
+    rng = np.random.default_rng(B + HKV)
+    K, G, D, PAGE = 2, 2, 64, 64
+    sl = rng.integers(1, 200, B).astype(np.int32)
+    sl[rng.permutation(B)[:long_ones]] = longest - rng.integers(0, 100, long_ones)
+    npg = -(-sl // PAGE)
+    pages = int(npg.sum())
+    kc, ks = O.quantize_fp4(rng.standard_normal((pages, HKV, PAGE, D)).astype(np.float32))
+    vc, vs = O.quantize_fp4(rng.standard_normal((pages, HKV, PAGE, D)).astype(np.float32))
+    bt = np.zeros((B, -(-width // PAGE)), np.int32)
+    perm, at = rng.permutation(pages).astype(np.int32), 0
+    for b in range(B):
+        bt[b, :npg[b]] = perm[at:at + npg[b]]
+        at += npg[b]
+    qb = O.bf16_bits(rng.standard_normal((B, K, HKV * G, D)).astype(np.float32))
+    n = uq_cuda.workspace_floats(B, K, HKV * G, HKV, D, nsplit)
+    ws = torch.full((n + 4096,), 7.0, device="cuda")
+    out = uq_cuda.uq_decode_cuda(dev(qb.view(np.int16), torch.bfloat16), *(dev(a) for a in (kc, ks, vc, vs, bt, sl)), nsplit=nsplit, workspace=ws)
+    assert uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
+    check_close(out.float().cpu().numpy(), O.reference(qb, kc, ks, vc, vs, bt, sl), f"nsplit={nsplit}")
+    assert bool((ws[n:] == 7.0).all())
