@@ -10,6 +10,7 @@ library is missing or the device is not CUDA, the call raises.
 """
 import ctypes
 import os
+import struct
 
 import torch
 
@@ -31,6 +32,9 @@ class UQParams(ctypes.Structure):
                 ("variant", ctypes.c_int), ("mb", ctypes.c_int), ("fmt", ctypes.c_int), ("k_ts", ctypes.c_float),
                 ("v_ts", ctypes.c_float)]
 
+
+_PARAMS = struct.Struct("=10Q8if3i2f")
+assert _PARAMS.size == ctypes.sizeof(UQParams)
 
 EXPORTS = ("uqb_block_m", "uqb_mo_elems", "uqb_ml_elems", "uqb_workspace_bytes", "uqb_decode_launch", "uqb_decode_launch_ws",
            "uqb_has_sm90", "uqb_append_launch", "uqb_append_ex_launch", "uqb_append_nvfp4_launch", "uqb_append_nvfp4_ex_launch", "uqb_fwht_launch", "uqb_decode_partial_launch", "uqb_tree_decode_launch", "uqb_merge_launch", "uqb_merge_packed_launch", "uqb_last_status",
@@ -111,7 +115,7 @@ class _on_device:
     microseconds; a serving loop is on its device already)."""
 
     def __init__(self, device):
-        self.ctx = None if device.index is None or device.index == torch.cuda.current_device() else torch.cuda.device(device)
+        self.ctx = None if device.index is None or device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
 
     def __enter__(self):
         if self.ctx is not None:
@@ -129,7 +133,7 @@ def _check(err, what):
 
 
 def _stream(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(t.device.index)   # (the integer alone: no Stream object per call)
 
 
 def _need_cuda(*ts):
@@ -140,13 +144,11 @@ def _need_cuda(*ts):
 
 def _params(q, kc, ks, vc, vs, bt, sl, nsplit, sm_scale, variant=0, mb=0, fmt=0, k_ts=1.0, v_ts=1.0):
     B, K, HQ, D = q.shape
-    p = UQParams()
-    p.q, p.kc, p.ks, p.vc, p.vs = q.data_ptr(), kc.data_ptr(), ks.data_ptr(), vc.data_ptr(), vs.data_ptr()
-    p.block_table, p.seq_lens = bt.data_ptr(), sl.data_ptr()
-    p.B, p.K, p.HQ, p.D = B, K, HQ, D
-    p.HKV, p.PAGE, p.max_pages, p.nsplit = kc.shape[1], kc.shape[2], bt.shape[1], int(nsplit)
-    p.sm_scale, p.variant, p.mb, p.fmt, p.k_ts, p.v_ts = float(sm_scale), int(variant), int(mb), int(fmt), float(k_ts), float(v_ts)
-    return p
+    kshape = kc.shape
+    # the structure's fields in its order, packed at once (a store per field is half of the call's arithmetic)
+    return UQParams.from_buffer_copy(_PARAMS.pack(q.data_ptr(), kc.data_ptr(), ks.data_ptr(), vc.data_ptr(), vs.data_ptr(), bt.data_ptr(), sl.data_ptr(),
+                                                  0, 0, 0, B, K, HQ, kshape[1], D, kshape[2], bt.shape[1], int(nsplit), float(sm_scale), int(variant),
+                                                  int(mb), int(fmt), float(k_ts), float(v_ts)))
 
 
 class _Ext:
@@ -313,7 +315,7 @@ def uq_tree_decode(q, kc, ks, vc, vs, block_table, seq_lens, tree_mask=None, *, 
     if out is None:
         out = torch.empty_like(q)
     p.mo, p.ml, p.out = workspace.data_ptr(), workspace.data_ptr() + 4 * n_mo, out.data_ptr()
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         err = L.uqb_tree_decode_launch(ctypes.byref(p), tm.data_ptr(), _stream(q))
     _check(err, "uq_tree_decode_launch")
     return out
@@ -339,7 +341,7 @@ def uq_decode_static(q, kc, ks, vc, vs, block_table, seq_lens, out, *, nsplit=No
     need, have = int(L.uqb_workspace_bytes(ctypes.byref(p))), int(L.uqb_static_scratch_bytes())
     if need > have:
         raise RuntimeError(f"this call needs {need} bytes of partials, the built-in scratch holds {have}: lower nsplit or pass a workspace to uq_decode_cuda")
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         err = L.uqb_decode_launch_static(ctypes.byref(p), 0, 0, _stream(q))
     _check(err, "uq_decode_launch_static")
     return out
@@ -373,7 +375,7 @@ def fwht(x, out=None):
     if out.shape != x.shape or out.dtype != x.dtype or not out.is_contiguous():
         raise RuntimeError("out must be contiguous with x's shape and dtype")
     D = x.shape[-1]
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         err = lib().uqb_fwht_launch(x.data_ptr(), out.data_ptr(), x.numel() // max(1, D), D, _DTYPE[x.dtype], _stream(x))
     _check(err, "uq_fwht_launch")
     return out
@@ -397,7 +399,7 @@ def append_kv(kc, ks, vc, vs, key, value, slot_mapping, *, rotate_k=False, rule=
     for t in (kc, ks, vc, vs):
         if not t.is_contiguous() or t.dtype != torch.uint8:
             raise RuntimeError("cache tensors must be contiguous uint8")
-    with torch.cuda.device(key.device):
+    with _on_device(key.device):
         err = lib().uqb_append_ex_launch(kc.data_ptr(), ks.data_ptr(), vc.data_ptr(), vs.data_ptr(), key.data_ptr(), value.data_ptr(),
                                          slots.data_ptr(), T, HKV, D, kc.shape[2], _DTYPE[key.dtype], flags, c, _stream(key))
     _check(err, "uq_append_launch")
@@ -421,7 +423,7 @@ def append_kv_nvfp4(kc, ks, vc, vs, key, value, slot_mapping, k_ts, v_ts, kernel
     for t in (kc, ks, vc, vs):
         if not t.is_contiguous() or t.dtype != torch.uint8:
             raise RuntimeError("cache tensors must be contiguous uint8")
-    with torch.cuda.device(key.device):
+    with _on_device(key.device):
         err = lib().uqb_append_nvfp4_ex_launch(kc.data_ptr(), ks.data_ptr(), vc.data_ptr(), vs.data_ptr(), key.data_ptr(), value.data_ptr(),
                                                slots.data_ptr(), T, HKV, D, kc.shape[2], _DTYPE[key.dtype], float(k_ts), float(v_ts),
                                                _KERNEL_FLAG[kernel], _stream(key))
@@ -477,7 +479,7 @@ def quantize_on_write(x, code, scale, slots, rule="ceil", c=None, kernel=None):
     N, HKV, D = x.shape
     x = x.contiguous()
     sl = slots.to(torch.int64).contiguous()
-    with torch.cuda.device(x.device):
+    with _on_device(x.device):
         err = lib().uqb_append_ex_launch(code.data_ptr(), scale.data_ptr(), None, None, x.data_ptr(), None, sl.data_ptr(),
                                          N, HKV, D, code.shape[2], _DTYPE[x.dtype], flags, c, _stream(x))
     _check(err, "uq_append_launch")
@@ -512,7 +514,7 @@ def uq_decode_partial(q, kc, ks, vc, vs, block_table, seq_lens, pos_offset=None,
         o = torch.empty(B, K, HQ, D, dtype=torch.float32, device=q.device)
         lse = torch.empty(B, K, HQ, dtype=torch.float32, device=q.device)
     po = None if pos_offset is None else pos_offset.to(torch.int32).contiguous()
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         err = L.uqb_decode_partial_launch(ctypes.byref(p), None if po is None else po.data_ptr(), o.data_ptr(), lse.data_ptr(), _stream(q))
     _check(err, "uq_decode_partial_launch")
     return o, lse
@@ -526,7 +528,7 @@ def uq_merge(o_parts, lse2_parts, out=None):
     rows = lse2_parts[0].numel()
     if out is None:
         out = torch.empty(o_parts.shape[1:], dtype=torch.bfloat16, device=o_parts.device)
-    with torch.cuda.device(o_parts.device):
+    with _on_device(o_parts.device):
         err = lib().uqb_merge_launch(o_parts.data_ptr(), lse2_parts.data_ptr(), R, rows, D, out.data_ptr(), _stream(o_parts))
     _check(err, "uq_merge_launch")
     return out
@@ -537,7 +539,7 @@ def uq_merge_packed(packed, rows, D, out):
     out bf16 [..., D] with rows rows.  Not in the reference."""
     _need_cuda(packed, out)
     packed = packed.contiguous()
-    with torch.cuda.device(packed.device):
+    with _on_device(packed.device):
         err = lib().uqb_merge_packed_launch(packed.data_ptr(), packed.shape[0], rows, D, out.data_ptr(), _stream(packed))
     _check(err, "uq_merge_packed_launch")
     return out
@@ -698,7 +700,7 @@ class ContextSplit:
             ws = self._ws[key] = (torch.empty(n_mo + n_ml, dtype=torch.float32, device=q.device), n_mo)
         p.mo, p.ml = ws[0].data_ptr(), ws[0].data_ptr() + 4 * ws[1]
         bases = (ctypes.c_void_p * self.world)(*self.bases)
-        with torch.cuda.device(q.device):
+        with _on_device(q.device):
             err = L.uqb_decode_partial_push_launch(ctypes.byref(p), pos_offset.data_ptr(), bases, self.world, self.rank, int(seq), _stream(q))
         _check(err, "uq_decode_partial_push_launch")
 
@@ -706,7 +708,7 @@ class ContextSplit:
         """Second launch of call `seq`: wait for every rank's flag, merge the slots of the local buffer into `out` (bf16, q's shape)."""
         B, K, HQ, D = q.shape
         out = torch.empty_like(q) if out is None else out
-        with torch.cuda.device(q.device):
+        with _on_device(q.device):
             err = lib().uqb_merge_wait_launch(self.bases[self.rank], self.world, int(seq), B * K * HQ, D, out.data_ptr(), self.wait_ns, _stream(q))
         _check(err, "uq_merge_wait_launch")
         return out

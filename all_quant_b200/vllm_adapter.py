@@ -61,12 +61,11 @@ def uq_verify_attention(query, kc, ks, vc, vs, block_table, seq_lens, K, *, sm_s
 
 
 def _slots_for(workspace, B, K, HQ, HKV, D, n_pages, device):
-    want = uq_cuda.auto_nsplit(B, HKV, n_pages, torch.cuda.get_device_properties(device).multi_processor_count, K, HQ // HKV)
-    while want > 1 and uq_cuda.workspace_floats(B, K, HQ, HKV, D, want) > workspace.numel():
-        want -= 1
-    if uq_cuda.workspace_floats(B, K, HQ, HKV, D, want) > workspace.numel():
+    want = uq_cuda.auto_nsplit(B, HKV, n_pages, uq_cuda._sm_count(device), K, HQ // HKV)
+    one = uq_cuda.workspace_floats(B, K, HQ, HKV, D, 1)   # (n slots take n times one slot's; 0 for arguments the launch refuses)
+    if one > workspace.numel():
         raise RuntimeError("scratch too small")
-    return want
+    return min(want, workspace.numel() // one) if one else want
 
 
 def append_kv(kc, ks, vc, vs, key, value, slot_mapping, *, rotate_k=False, rule="ceil", c=None, kernel=None):
