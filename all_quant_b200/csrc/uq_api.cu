@@ -4,7 +4,7 @@
 // Dispatch (the reference's is a template tree over variant / BLOCK_M / warps / stages, reference
 // cuda/uq_decode.cu:402-626; this library has two kernels and ignores those hints):
 //   tcgen05 kernel  when head_dim, page size, alignment and row count are ones it serves (uq_verify_tc.cu): every
-//                   page size that is a multiple of 16 from 16 to 1024 tokens, up to 64 rows per launch, 65-128 rows as draft chunks
+//                   page size that is a multiple of 16 from 16 to 1024 tokens, up to 64 rows per work item, 65-128 rows as two chunks of drafts
 //   CUDA-core kernel for everything else (uq_verify_fma.cu)
 // followed by the combine kernel.  Every check happens before the first launch, so
 // cudaErrorInvalidValue means nothing was enqueued (callers of the reference skip on it).
@@ -144,7 +144,7 @@ cudaError_t run(const UQParams& p, const int32_t* pos_offset, float* o_part, flo
   return run_one(p, x, o_part, lse_part, s, push);
 }
 
-// One launch of a verify kernel and its combine; x carries the caller's pointers and the draft chunk.
+// The launch of a verify kernel and its combine; x carries the caller's pointers.
 cudaError_t run_one(const UQParams& p, UQLaunch x, float* o_part, float* lse_part, cudaStream_t s, const UQPeerPush* push) {
   x.G = p.HQ / p.HKV;
   x.chunks = 1;
@@ -157,7 +157,7 @@ cudaError_t run_one(const UQParams& p, UQLaunch x, float* o_part, float* lse_par
   const int forced = forced_path();
   // More query rows than the tensor-core kernel's tile takes (up to the 128 of uq_block_m): the drafts run as two chunks of one
   // launch.  As two launches, one after the other in the same scratch, start-up, combine and an underfilled chip were paid
-  // twice: B=4, 8 K tokens, 16 drafts at a group of 8 took 61 us, 45 in one launch.
+  // twice: B=4, 4-8 K tokens, 16 drafts at a group of 8 took 60 us of GPU time, 41 in one launch.
   UQLaunch xc = x;
   if (x.rows > 64 && x.G <= 64) {
     const int fit = 64 / x.G;

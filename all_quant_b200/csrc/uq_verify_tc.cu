@@ -28,7 +28,8 @@
 //                          128-byte-swizzled fp16 tile in shared memory (ring of 2); gives its raw stage back as soon as the
 //                          key's codes and scale bytes are in registers.
 //   copy      2 warps      (K side / V side of every tile) TMA tensor copies of the code pages + bulk copies of the scale
-//                          pages into a ring of raw stages (3 at head_dim 128), mbarrier complete_tx.  No multicast.
+//                          pages into a ring of raw stages (3 at head_dim 128), mbarrier complete_tx.  No multicast.  Small pages
+//                          and head_dim 64 (dispatch_rows): a third warp brings the scale slices by per-lane asynchronous copies.
 //   issue     1 thread     chosen by elect.sync: P.V of tile i, then Q.K of tile i + 2; tcgen05.commit to mbarriers; owns the
 //                          TMEM allocation.
 // Work is a flat list of tiles over all (sequence, kv head) items, cut into chunks of equal WEIGHT (an item counts its tiles
