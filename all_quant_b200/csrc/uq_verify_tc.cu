@@ -795,11 +795,13 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   uint32_t* redo = reinterpret_cast<uint32_t*>(sm + C::oRedo);
   int* chunk_s = reinterpret_cast<int*>(sm + C::oChunk);
   for (int i = tid; i <= kRedoWords; i += kThreads) redo[i] = 0u;
+  uq_pdl_wait();   // from here on global memory is read and written
+  // (the tensor memory is taken only now: a block of the kernel before this one may sit on the same SM, release its dependents and
+  // allocate afterwards, and would wait for columns that this CTA held while it waited for that block)
   if (warp == kWarpMma) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sm_a + C::oTmemSlot) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  uq_pdl_wait();   // from here on global memory is read and written
   {
     // the queries (B x K x Hq x D bf16, read once per segment by whichever CTA gets it) go to L2 now, a slice per CTA, while
     // the set-up below runs: the first segment's conversion and every later one then find them there

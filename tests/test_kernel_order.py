@@ -1,0 +1,32 @@
+"""What every kernel launched as a programmatic dependent has to keep to, checked on the sources (no GPU): such a kernel starts while
+its predecessor on the stream is still running, so before its wait it may neither touch memory nor hold what the predecessor needs."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "all_quant_b200", "csrc")
+
+
+def kernels(name):
+    """{kernel: body} of a source file, comments taken out."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+    out = {}
+    for m in re.finditer(r"__global__[^;{]*?\b(uq_\w+_kernel)\s*\(", text):
+        at = text.index("{", m.end())
+        depth, end = 0, at
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[end], 0)
+            if depth == 0:
+                break
+            end += 1
+        out[m.group(1)] = text[at:end + 1]
+    return out
+
+
+def test_tensor_memory_is_allocated_after_the_wait():
+    """A block that held all 512 columns while it waits for the kernel before it would starve a block of that kernel on the same SM
+    that lets its successor go first and allocates tensor memory afterwards: each would wait for the other."""
+    body = kernels("uq_verify_tc.cu")["uq_verify_tc_kernel"]
+    wait = [m.end() for m in re.finditer(r"uq_pdl_wait\w*\(", body)]
+    alloc = body.index("tcgen05.alloc")
+    assert len(wait) == 2 and body.count("tcgen05.alloc") == 1   # (the first one is that of the early exit on a misplaced buffer)
+    assert "return;" in body[wait[0]:wait[1]] and alloc > wait[1]
