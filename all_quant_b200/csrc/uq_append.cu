@@ -135,9 +135,9 @@ __global__ void __launch_bounds__(128) uq_append_kernel(uint8_t* __restrict__ kc
                                                         const int64_t* __restrict__ slots, int T_tok, int HKV, int D, int PAGE, int nstream,
                                                         int flags, float c) {
   uq_pdl_release();
-  uq_pdl_wait();
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  const unsigned tid = uq_pdl_wait_index();
+  const int warp = (blockIdx.x * blockDim.x + tid) >> 5;
+  const int lane = tid & 31;
   const int total = T_tok * HKV * nstream;
   if (warp >= total) return;
   const int stream = warp % nstream;
@@ -351,15 +351,15 @@ __global__ void __launch_bounds__(256) uq_append_bulk_kernel(uint8_t* __restrict
                                                              const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
                                                              int PAGE, int page_shift, int paper, float c) {
   uq_pdl_release();
-  uq_pdl_wait();
+  const unsigned tid = uq_pdl_wait_index();
   constexpr bool kExactTies = sizeof(T) == 4;   // fp32 inputs can sit anywhere: half-way values are corrected by comparison
   constexpr int NP = bulk_pieces<T>();          // pieces per thread: 128 bytes of input in flight
   const int stream = blockIdx.y;
   const T* __restrict__ src = stream ? value : key;
   uint8_t* __restrict__ codes = stream ? vc : kc;
   uint8_t* __restrict__ scales = stream ? vs : ks;
-  const int lane = threadIdx.x & 31;
-  const uint32_t wp0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32u * NP);   // the warp's first piece (8 channels)
+  const int lane = tid & 31;
+  const uint32_t wp0 = (blockIdx.x * (blockDim.x >> 5) + (tid >> 5)) * (32u * NP);   // the warp's first piece (8 channels)
   const uint32_t p0 = wp0 + lane;                                                            // this lane's first piece
   const int ppr_shift = D == 64 ? 3 : (D == 128 ? 4 : 5);   // pieces per row = D / 8
   Piece<T> pc[NP];
@@ -486,9 +486,9 @@ __global__ void __launch_bounds__(128) uq_append_nvfp4_kernel(uint8_t* __restric
                                                               const int64_t* __restrict__ slots, int T_tok, int HKV, int D, int PAGE, float k_ts,
                                                               float v_ts) {
   uq_pdl_release();
-  uq_pdl_wait();
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  const unsigned tid = uq_pdl_wait_index();
+  const int warp = (blockIdx.x * blockDim.x + tid) >> 5;
+  const int lane = tid & 31;
   if (warp >= T_tok * HKV * 2) return;
   const int stream = warp & 1;
   const int h = (warp >> 1) % HKV;
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(256) uq_append_nvfp4_bulk_kernel(uint8_t* __re
                                                                    const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
                                                                    int PAGE, int page_shift, float k_ts, float v_ts) {
   uq_pdl_release();
-  uq_pdl_wait();
+  const unsigned tid = uq_pdl_wait_index();
   constexpr int NP = bulk_pieces<T>();
   constexpr bool kAddZero = sizeof(T) == 4;   // fp32 inputs: any product can underflow, +0 is added after the multiplication
   // a 16-bit input's smallest non-zero magnitude (2^-133 bf16, 2^-24 fp16) times the reciprocal stays a normal number
@@ -581,8 +581,8 @@ __global__ void __launch_bounds__(256) uq_append_nvfp4_bulk_kernel(uint8_t* __re
   uint8_t* __restrict__ codes = stream ? vc : kc;
   uint8_t* __restrict__ scales = stream ? vs : ks;
   const float ts = stream ? v_ts : k_ts;
-  const int lane = threadIdx.x & 31;
-  const uint32_t wp0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32u * NP);
+  const int lane = tid & 31;
+  const uint32_t wp0 = (blockIdx.x * (blockDim.x >> 5) + (tid >> 5)) * (32u * NP);
   const uint32_t p0 = wp0 + lane;
   const int ppr_shift = D == 64 ? 3 : (D == 128 ? 4 : 5);
   Piece<T> pc[NP];
@@ -688,9 +688,9 @@ bool bulk_nvfp4_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const
 template <typename T>
 __global__ void __launch_bounds__(128) uq_fwht_kernel(const T* __restrict__ x, T* __restrict__ out, long long rows, int D) {
   uq_pdl_release();
-  uq_pdl_wait();
-  const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  const unsigned tid = uq_pdl_wait_index();
+  const long long row = ((long long)blockIdx.x * blockDim.x + tid) >> 5;
+  const int lane = tid & 31;
   if (row >= rows) return;
   float xs[2][4];
 #pragma unroll

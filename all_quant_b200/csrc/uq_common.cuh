@@ -18,6 +18,14 @@
 // touches global memory before it.  uq_pdl_release() lets the next kernel be set up as soon as all blocks of this one have
 // started.  Both are no-ops in an ordinary launch.
 UQ_DEV void uq_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The wait, and the thread's index as a value that exists only from there on.  Loads through const __restrict__ pointers and __ldg are
+// loads of memory that does not change while the kernel runs, which the compiler may move upwards across the wait; with an address
+// made of this index there is nothing to load from before it.
+UQ_DEV unsigned uq_pdl_wait_index() {
+  unsigned t = threadIdx.x;
+  asm volatile("griddepcontrol.wait;" : "+r"(t)::"memory");
+  return t;
+}
 UQ_DEV void uq_pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
 inline cudaError_t uq_launch(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, bool dependent, A... args) {

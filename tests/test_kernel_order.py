@@ -30,3 +30,15 @@ def test_tensor_memory_is_allocated_after_the_wait():
     alloc = body.index("tcgen05.alloc")
     assert len(wait) == 2 and body.count("tcgen05.alloc") == 1   # (the first one is that of the early exit on a misplaced buffer)
     assert "return;" in body[wait[0]:wait[1]] and alloc > wait[1]
+
+
+def test_indexes_of_read_only_loads_come_out_of_the_wait():
+    """What is read through a const __restrict__ pointer or __ldg counts as unchanged during the whole kernel, so the compiler may
+    move such a load above the wait - where the kernel before it may still be writing.  In the kernels that read their inputs this
+    way every address is made of a thread index that the wait itself returns."""
+    bodies = kernels("uq_append.cu")
+    assert len(bodies) == 5
+    for name, body in bodies.items():
+        assert body.count("uq_pdl_wait_index()") == 1 and "threadIdx" not in body, name
+        wait = body.index("uq_pdl_wait_index()")
+        assert not re.search(r"\b(key|value|slots|src|x)\s*\[|__ldg|\.load\(", body[:wait]), name
