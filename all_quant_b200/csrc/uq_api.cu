@@ -37,7 +37,7 @@ cudaError_t uq_verify_fma_dispatch(const UQParams&, const UQLaunch&, cudaStream_
 cudaError_t uq_verify_tc_dispatch(const UQParams&, const UQLaunch&, cudaStream_t);
 bool uq_verify_tc_serves(const UQParams&, const UQLaunch&);
 int uq_verify_tc_splits(const UQParams&, const UQLaunch&);
-cudaError_t uq_combine_dispatch(const UQParams&, const UQLaunch&, float*, float*, const UQPeerPush*, bool, cudaStream_t);
+cudaError_t uq_combine_dispatch(const UQParams&, const UQLaunch&, float*, float*, const UQPeerPush*, cudaStream_t);
 cudaError_t uq_merge_wait_dispatch(const void*, int, size_t, unsigned int, size_t, int, void*, unsigned long long, unsigned int*, cudaStream_t);
 cudaError_t uq_merge_dispatch(const float*, const float*, int, size_t, int, void*, cudaStream_t);
 cudaError_t uq_layout_dispatch(int, uint8_t*, uint8_t*, uint8_t*, uint8_t*, uint8_t*, long long, int, int, int, int, int, cudaStream_t);
@@ -171,9 +171,7 @@ cudaError_t run_one(const UQParams& p, UQLaunch x, float* o_part, float* lse_par
   cudaError_t e;
   const bool timed = t_ev_before && t_ev_after;
   if (timed) cudaEventRecord(t_ev_before, s);
-  // (UQ_B200_CFG="pdl=0" turns programmatic dependent launches off; an event between two launches needs them apart)
-  static const bool pdl_on = !(std::getenv("UQ_B200_CFG") && std::strstr(std::getenv("UQ_B200_CFG"), "pdl=0"));
-  x.pdl = tc && pdl_on && !timed;
+  x.pdl = tc && uq_pdl_on() && !timed;   // (an event between two launches needs them apart)
   if (tc) {
     x.ns_eff = uq_verify_tc_splits(p, x);
     e = uq_verify_tc_dispatch(p, x, s);
@@ -188,7 +186,7 @@ cudaError_t run_one(const UQParams& p, UQLaunch x, float* o_part, float* lse_par
   if (timed) cudaEventRecord(t_ev_after, s);
   if (e != cudaSuccess) return e;
   g_launches += 2;
-  return uq_combine_dispatch(p, x, o_part, lse_part, push, x.pdl != 0, s);
+  return uq_combine_dispatch(p, x, o_part, lse_part, push, s);
 }
 
 }  // namespace

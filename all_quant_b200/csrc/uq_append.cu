@@ -133,8 +133,8 @@ template <typename T>
 __global__ void __launch_bounds__(128) uq_append_kernel(uint8_t* __restrict__ kc, uint8_t* __restrict__ ks, uint8_t* __restrict__ vc,
                                                         uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                         const int64_t* __restrict__ slots, int T_tok, int HKV, int D, int PAGE, int nstream,
-                                                        int flags, float c) {
-  uq_pdl_release();
+                                                        int flags, float c, int pdl) {
+  if (pdl) uq_pdl_release();
   const unsigned tid = uq_pdl_wait_index();
   const int warp = (blockIdx.x * blockDim.x + tid) >> 5;
   const int lane = tid & 31;
@@ -349,8 +349,8 @@ template <typename T, bool kRot>
 __global__ void __launch_bounds__(256) uq_append_bulk_kernel(uint8_t* __restrict__ kc, uint8_t* __restrict__ ks, uint8_t* __restrict__ vc,
                                                              uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                              const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
-                                                             int PAGE, int page_shift, int paper, float c) {
-  uq_pdl_release();
+                                                             int PAGE, int page_shift, int paper, float c, int pdl) {
+  if (pdl) uq_pdl_release();
   const unsigned tid = uq_pdl_wait_index();
   constexpr bool kExactTies = sizeof(T) == 4;   // fp32 inputs can sit anywhere: half-way values are corrected by comparison
   constexpr int NP = bulk_pieces<T>();          // pieces per thread: 128 bytes of input in flight
@@ -468,11 +468,12 @@ bool bulk_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const T* ke
   int shift = -1;
   if ((PAGE & (PAGE - 1)) == 0) { shift = 0; while ((1 << shift) < PAGE) shift++; }
   const unsigned per_block = (UQ_BULK_THREADS / 32u) * 32u * bulk_pieces<T>();
+  const bool pdl = uq_pdl_on();
   const dim3 grid((unsigned)((np + per_block - 1) / per_block), (unsigned)nstream);
   if (flags & kRotateK)
-    uq_launch(uq_append_bulk_kernel<T, true>, grid, UQ_BULK_THREADS, 0, s, true, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c);
+    uq_launch(uq_append_bulk_kernel<T, true>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c, (int)pdl);
   else
-    uq_launch(uq_append_bulk_kernel<T, false>, grid, UQ_BULK_THREADS, 0, s, true, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c);
+    uq_launch(uq_append_bulk_kernel<T, false>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c, (int)pdl);
   return true;
 }
 
@@ -484,8 +485,8 @@ template <typename T>
 __global__ void __launch_bounds__(128) uq_append_nvfp4_kernel(uint8_t* __restrict__ kc, uint8_t* __restrict__ ks, uint8_t* __restrict__ vc,
                                                               uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                               const int64_t* __restrict__ slots, int T_tok, int HKV, int D, int PAGE, float k_ts,
-                                                              float v_ts) {
-  uq_pdl_release();
+                                                              float v_ts, int pdl) {
+  if (pdl) uq_pdl_release();
   const unsigned tid = uq_pdl_wait_index();
   const int warp = (blockIdx.x * blockDim.x + tid) >> 5;
   const int lane = tid & 31;
@@ -568,8 +569,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) uq_append_nvfp4_bulk_kernel(uint8_t* __restrict__ kc, uint8_t* __restrict__ ks, uint8_t* __restrict__ vc,
                                                                    uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                                    const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
-                                                                   int PAGE, int page_shift, float k_ts, float v_ts) {
-  uq_pdl_release();
+                                                                   int PAGE, int page_shift, float k_ts, float v_ts, int pdl) {
+  if (pdl) uq_pdl_release();
   const unsigned tid = uq_pdl_wait_index();
   constexpr int NP = bulk_pieces<T>();
   constexpr bool kAddZero = sizeof(T) == 4;   // fp32 inputs: any product can underflow, +0 is added after the multiplication
@@ -679,15 +680,16 @@ bool bulk_nvfp4_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const
   int shift = -1;
   if ((PAGE & (PAGE - 1)) == 0) { shift = 0; while ((1 << shift) < PAGE) shift++; }
   const unsigned per_block = (UQ_BULK_THREADS / 32u) * 32u * bulk_pieces<T>();
+  const bool pdl = uq_pdl_on();
   const dim3 grid((unsigned)((np + per_block - 1) / per_block), 2u);
-  uq_launch(uq_append_nvfp4_bulk_kernel<T>, grid, UQ_BULK_THREADS, 0, s, true, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, k_ts, v_ts);
+  uq_launch(uq_append_nvfp4_bulk_kernel<T>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, k_ts, v_ts, (int)pdl);
   return true;
 }
 
 // The transform alone (the queries of a cache whose keys were rotated): one warp per row, out may be x.
 template <typename T>
-__global__ void __launch_bounds__(128) uq_fwht_kernel(const T* __restrict__ x, T* __restrict__ out, long long rows, int D) {
-  uq_pdl_release();
+__global__ void __launch_bounds__(128) uq_fwht_kernel(const T* __restrict__ x, T* __restrict__ out, long long rows, int D, int pdl) {
+  if (pdl) uq_pdl_release();
   const unsigned tid = uq_pdl_wait_index();
   const long long row = ((long long)blockIdx.x * blockDim.x + tid) >> 5;
   const int lane = tid & 31;
@@ -715,11 +717,12 @@ cudaError_t uq_fwht_dispatch(const void* x, void* out, long long rows, int D, in
   if (rows == 0) return cudaSuccess;
   if (!x || !out || rows < 0 || !(D == 64 || D == 128 || D == 256) || dtype < 0 || dtype > 2) return cudaErrorInvalidValue;
   const long long blocks = (rows + 3) / 4;
+  const bool pdl = uq_pdl_on();
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
   switch (dtype) {
-    case 0: uq_launch(uq_fwht_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, true, (const float*)x, (float*)out, rows, D); break;
-    case 1: uq_launch(uq_fwht_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, true, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, D); break;
-    default: uq_launch(uq_fwht_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, true, (const __half*)x, (__half*)out, rows, D); break;
+    case 0: uq_launch(uq_fwht_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const float*)x, (float*)out, rows, D, (int)pdl); break;
+    case 1: uq_launch(uq_fwht_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, D, (int)pdl); break;
+    default: uq_launch(uq_fwht_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const __half*)x, (__half*)out, rows, D, (int)pdl); break;
   }
   return cudaGetLastError();
 }
@@ -743,10 +746,11 @@ cudaError_t uq_append_nvfp4_dispatch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint
     if (route == kRouteBulk) return cudaErrorInvalidValue;
   }
   const int blocks = (int)((warps + 3) / 4);
+  const bool pdl = uq_pdl_on();
   switch (dtype) {
-    case 0: uq_launch(uq_append_nvfp4_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
-    case 1: uq_launch(uq_append_nvfp4_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
-    default: uq_launch(uq_append_nvfp4_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts); break;
+    case 0: uq_launch(uq_append_nvfp4_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
+    case 1: uq_launch(uq_append_nvfp4_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
+    default: uq_launch(uq_append_nvfp4_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
   }
   return cudaGetLastError();
 }
@@ -778,10 +782,11 @@ cudaError_t uq_append_dispatch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* v
     if (route == kRouteBulk) return cudaErrorInvalidValue;   // asked for by name and not served (alignment, size)
   }
   const int blocks = (int)((warps + 3) / 4);
+  const bool pdl = uq_pdl_on();
   switch (dtype) {
-    case 0: uq_launch(uq_append_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
-    case 1: uq_launch(uq_append_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
-    default: uq_launch(uq_append_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, true, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c); break;
+    case 0: uq_launch(uq_append_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
+    case 1: uq_launch(uq_append_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
+    default: uq_launch(uq_append_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
   }
   return cudaGetLastError();
 }

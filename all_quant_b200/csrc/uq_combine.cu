@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(128) uq_combine_kernel(const UQParams p, const
   const int lane = threadIdx.x & 31;
   const int total = p.B * p.K * p.HQ;
   // (nothing of the partials is read before the whole attention grid has completed and its writes are visible)
-  if (gridDim.x <= kReleaseBlocks) uq_pdl_release();
+  if (x.pdl && gridDim.x <= kReleaseBlocks) uq_pdl_release();
   uq_pdl_wait();
   if (row < total) {
   const int h = row % p.HQ, j = (row / p.HQ) % p.K, b = row / (p.HQ * p.K);
@@ -198,15 +198,15 @@ __global__ void __launch_bounds__(128) uq_merge_kernel(const float* o, const flo
 
 }  // namespace
 
-cudaError_t uq_combine_dispatch(const UQParams& p, const UQLaunch& x, float* o_part, float* lse_part, const UQPeerPush* push, bool pdl, cudaStream_t s) {
+cudaError_t uq_combine_dispatch(const UQParams& p, const UQLaunch& x, float* o_part, float* lse_part, const UQPeerPush* push, cudaStream_t s) {
   const int rows = p.B * p.K * p.HQ;
   if (rows == 0) return cudaSuccess;
   const UQPeerPush none{};
   const dim3 grid((rows + 3) / 4);
   float* no_f = nullptr;
-  if (push) return uq_launch(uq_combine_kernel<2>, grid, 128u, 0, s, pdl, p, x, no_f, no_f, *push);
-  if (o_part) return uq_launch(uq_combine_kernel<1>, grid, 128u, 0, s, pdl, p, x, o_part, lse_part, none);
-  return uq_launch(uq_combine_kernel<0>, grid, 128u, 0, s, pdl, p, x, no_f, no_f, none);
+  if (push) return uq_launch(uq_combine_kernel<2>, grid, 128u, 0, s, x.pdl != 0, p, x, no_f, no_f, *push);
+  if (o_part) return uq_launch(uq_combine_kernel<1>, grid, 128u, 0, s, x.pdl != 0, p, x, o_part, lse_part, none);
+  return uq_launch(uq_combine_kernel<0>, grid, 128u, 0, s, x.pdl != 0, p, x, no_f, no_f, none);
 }
 
 cudaError_t uq_merge_dispatch(const float* o, const float* lse, int R, size_t rows, int D, void* out, cudaStream_t s) {

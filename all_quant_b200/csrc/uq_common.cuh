@@ -2,6 +2,8 @@
 // caller's scratch, and the status record that bounded waits write to.
 #pragma once
 #include <cstdint>
+#include <cstdlib>
+#include <cstring>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -11,12 +13,13 @@
 #define UQ_DEV __device__ __forceinline__
 
 // ---- programmatic dependent launch ------------------------------------------------------------------
-// Every kernel of a call's chain (append, rotate, verify, combine) is launched as a programmatic dependent of what precedes it
-// on the stream: its blocks may be set up while that kernel's last blocks still run.  uq_pdl_wait() returns once everything
+// The append, rotate, tensor-core verify and (behind that) combine kernels are launched as programmatic dependents of what precedes
+// them on the stream: their blocks may be set up while that kernel's last blocks still run.  uq_pdl_wait() returns once everything
 // before it on the stream has completed with its writes visible; every block of every such kernel executes it (a grid whose
 // blocks left without it could complete before its predecessor, and the kernel after it would start too early), and none
 // touches global memory before it.  uq_pdl_release() lets the next kernel be set up as soon as all blocks of this one have
-// started.  Both are no-ops in an ordinary launch.
+// executed it (or left); the kernels execute it only when they are launched as dependents themselves, so that with the switch
+// below off a launch is an ordinary one for its neighbours on both sides.
 UQ_DEV void uq_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The wait, and the thread's index as a value that exists only from there on.  Loads through const __restrict__ pointers and __ldg are
 // loads of memory that does not change while the kernel runs, which the compiler may move upwards across the wait; with an address
@@ -27,6 +30,11 @@ UQ_DEV unsigned uq_pdl_wait_index() {
   return t;
 }
 UQ_DEV void uq_pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// UQ_B200_CFG="pdl=0" (read at the first launch) makes every launch of the library an ordinary one.
+inline bool uq_pdl_on() {
+  static const bool on = !(std::getenv("UQ_B200_CFG") && std::strstr(std::getenv("UQ_B200_CFG"), "pdl=0"));
+  return on;
+}
 template <typename... P, typename... A>
 inline cudaError_t uq_launch(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, bool dependent, A... args) {
   cudaLaunchConfig_t cfg{};

@@ -1677,7 +1677,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   UQ_TRACE_CTA_V(6, seg_i)
   // Not before here: released at its start, the combine's blocks crowd onto the first SMs that fall free (one sequence of 131 K
   // tokens at head_dim 256: 86.5 us a call, 78.9 with the release at the end of the CTA).
-  uq_pdl_release();
+  if (x.pdl) uq_pdl_release();
   // ---- common exit: TMEM goes back before the CTA ends
   if (warp == kWarpMma) {
     tc_fence_after();

@@ -1,5 +1,9 @@
 """Parity of the CUDA verify/decode attention with the reference's known answers and with the CPU oracle,
 through the C ABI (all_quant_b200.uq_cuda -> libuq_b200.so).  Needs a B200."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -410,3 +414,45 @@ def test_items_cut_into_no_more_pieces_than_they_have_slots(B, HKV, long_ones, l
     assert uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
     check_close(out.float().cpu().numpy(), O.reference(qb, kc, ks, vc, vs, bt, sl), f"nsplit={nsplit}")
     assert bool((ws[n:] == 7.0).all())
+
+
+CAPTURED_CHAIN = """
+import ctypes, torch
+from all_quant_b200 import uq_cuda
+B, K, HQ, HKV, D, PAGE, T = 2, 2, 8, 2, 64, 16, 40
+dev = dict(device="cuda")
+new = lambda row: torch.zeros(8, HKV, PAGE, row, dtype=torch.uint8, **dev)
+uq, nv = (new(D // 2), new(D // 32), new(D // 2), new(D // 32)), (new(D // 2), new(D // 16), new(D // 2), new(D // 16))
+key, slots = torch.randn(T, HKV, D, **dev).bfloat16(), torch.arange(T, **dev)
+q, r, out = (torch.randn(B, K, HQ, D, **dev).bfloat16() for _ in range(3))
+bt, sl = torch.arange(8, dtype=torch.int32, **dev).view(B, 4), torch.tensor([33, 7], dtype=torch.int32, **dev)
+ws = torch.empty(uq_cuda.workspace_floats(B, K, HQ, HKV, D, 4), **dev)
+
+def chain():
+    for kernel in ("rows", "bulk"):
+        uq_cuda.append_kv(*uq, key, key, slots, kernel=kernel)
+        uq_cuda.append_kv_nvfp4(*nv, key, key, slots, 0.1, 0.1, kernel=kernel)
+    uq_cuda.fwht(q, out=r)
+    uq_cuda.uq_decode_cuda(r, *uq, bt, sl, nsplit=4, workspace=ws, out=out)
+
+chain()
+torch.cuda.synchronize()
+cu, s, g, n = ctypes.CDLL("libcuda.so.1"), torch.cuda.Stream(), ctypes.c_void_p(), ctypes.c_size_t()
+assert cu.cuStreamBeginCapture_v2(ctypes.c_void_p(s.cuda_stream), 2) == 0
+with torch.cuda.stream(s):
+    chain()
+assert cu.cuStreamEndCapture(ctypes.c_void_p(s.cuda_stream), ctypes.byref(g)) == 0
+assert cu.cuGraphGetEdges_v2(g, None, None, None, ctypes.byref(n)) == 0
+ends, kind = [(ctypes.c_void_p * n.value)() for _ in range(2)], (ctypes.c_uint8 * (8 * n.value))()   # kind: 8 bytes per edge, byte 2 its type
+assert cu.cuGraphGetEdges_v2(g, ends[0], ends[1], kind, ctypes.byref(n)) == 0
+print("edges", n.value, "programmatic", sum(kind[8 * i + 2] == 1 for i in range(n.value)))
+"""
+
+
+@pytest.mark.parametrize("cfg,programmatic", [("", 6), ("pdl=0", 0)])
+def test_the_switch_makes_every_launch_an_ordinary_one(cfg, programmatic):
+    """Four appends, a rotation and a verify call with its combine, captured: all six edges between the seven kernels are
+    programmatic, and none with the switch off (read once per process, so each side is a process of its own)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CAPTURED_CHAIN], cwd=root, env={**os.environ, "UQ_B200_CFG": cfg}, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and f"edges 6 programmatic {programmatic}" in r.stdout, r.stdout + r.stderr
