@@ -107,3 +107,19 @@ def test_out_of_range_arguments_are_refused_and_sizes_do_not_wrap(over):
     # the size helpers return (no endless loop, no wrapped product): zero elements for arguments outside the served ranges
     assert L.uqb_workspace_bytes(ctypes.byref(p)) < (1 << 62)
     assert L.uqb_block_m(1 << 30, 1 << 30, 1) == 1 << 30
+
+
+@pytest.mark.parametrize("kw", [{}, {"sm_scale": 1e39}, {"sm_scale": -1e39}, {"k_ts": 1e300, "fmt": 1}, {"v_ts": float("inf")}, {"nsplit": (1 << 33) + 5},
+                                {"variant": -1, "mb": (1 << 31) + 7}, {"fmt": 1 << 40}])
+def test_parameters_beyond_their_fields_become_what_a_store_makes_of_them(kw):
+    """The parameter block packed in one step holds what storing field by field holds: a scale beyond fp32 is infinite, an integer
+    beyond 32 bits loses its upper ones, and the library then answers for the value (nothing is refused on the way)."""
+    import torch
+    q, c, t = torch.zeros(2, 3, 8, 64), torch.zeros(5, 4, 16, 32, dtype=torch.uint8), torch.zeros(2, 7, dtype=torch.int32)
+    a = {"nsplit": 4, "sm_scale": 0.125, "variant": 1, "mb": 2, "fmt": 0, "k_ts": 0.5, "v_ts": 0.25, **kw}
+    got = uq_cuda._params(q, c, c, c, c, t, t, **a)
+    want = uq_cuda.UQParams()
+    for f, v in {"q": q.data_ptr(), "kc": c.data_ptr(), "ks": c.data_ptr(), "vc": c.data_ptr(), "vs": c.data_ptr(), "block_table": t.data_ptr(),
+                 "seq_lens": t.data_ptr(), "B": 2, "K": 3, "HQ": 8, "D": 64, "HKV": 4, "PAGE": 16, "max_pages": 7, **a}.items():
+        setattr(want, f, v)
+    assert bytes(got) == bytes(want)
