@@ -457,10 +457,10 @@ __global__ void __launch_bounds__(256) uq_append_bulk_kernel(uint8_t* __restrict
   else encode(std::false_type{});
 }
 
-// the bulk kernel serves: pointers aligned for the vector loads, piece count within 32 bits
+// the bulk kernel serves: pointers aligned for the vector loads, piece count within 32 bits (false: not served, nothing launched; e: of the launch)
 template <typename T>
 bool bulk_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const T* key, const T* value, const int64_t* slots, int T_tok, int HKV,
-                 int D, int PAGE, int nstream, int flags, float c, cudaStream_t s) {
+                 int D, int PAGE, int nstream, int flags, float c, cudaStream_t s, cudaError_t& e) {
   const unsigned long long np = (unsigned long long)T_tok * HKV * (D / 8);
   const uintptr_t al = 15;
   if (np >= (1ull << 31) || ((reinterpret_cast<uintptr_t>(key) | reinterpret_cast<uintptr_t>(value)) & al)) return false;
@@ -471,9 +471,9 @@ bool bulk_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const T* ke
   const bool pdl = uq_pdl_on();
   const dim3 grid((unsigned)((np + per_block - 1) / per_block), (unsigned)nstream);
   if (flags & kRotateK)
-    uq_launch(uq_append_bulk_kernel<T, true>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c, (int)pdl);
+    e = uq_launch(uq_append_bulk_kernel<T, true>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c, (int)pdl);
   else
-    uq_launch(uq_append_bulk_kernel<T, false>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c, (int)pdl);
+    e = uq_launch(uq_append_bulk_kernel<T, false>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, (flags & kPaperRule) ? 1 : 0, c, (int)pdl);
   return true;
 }
 
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(256) uq_append_nvfp4_bulk_kernel(uint8_t* __re
 
 template <typename T>
 bool bulk_nvfp4_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const T* key, const T* value, const int64_t* slots, int T_tok, int HKV,
-                       int D, int PAGE, float k_ts, float v_ts, cudaStream_t s) {
+                       int D, int PAGE, float k_ts, float v_ts, cudaStream_t s, cudaError_t& e) {
   const unsigned long long np = (unsigned long long)T_tok * HKV * (D / 8);
   if (np >= (1ull << 31) || ((reinterpret_cast<uintptr_t>(key) | reinterpret_cast<uintptr_t>(value)) & 15)) return false;
   const uint32_t magic = HKV == 1 ? 0xffffffffu : (uint32_t)((1ull << 32) / (unsigned)HKV);
@@ -682,7 +682,7 @@ bool bulk_nvfp4_launch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* vs, const
   const unsigned per_block = (UQ_BULK_THREADS / 32u) * 32u * bulk_pieces<T>();
   const bool pdl = uq_pdl_on();
   const dim3 grid((unsigned)((np + per_block - 1) / per_block), 2u);
-  uq_launch(uq_append_nvfp4_bulk_kernel<T>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, k_ts, v_ts, (int)pdl);
+  e = uq_launch(uq_append_nvfp4_bulk_kernel<T>, grid, UQ_BULK_THREADS, 0, s, pdl, kc, ks, vc, vs, key, value, slots, (uint32_t)np, HKV, magic, D, PAGE, shift, k_ts, v_ts, (int)pdl);
   return true;
 }
 
@@ -719,12 +719,13 @@ cudaError_t uq_fwht_dispatch(const void* x, void* out, long long rows, int D, in
   const long long blocks = (rows + 3) / 4;
   const bool pdl = uq_pdl_on();
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
+  cudaError_t e;
   switch (dtype) {
-    case 0: uq_launch(uq_fwht_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const float*)x, (float*)out, rows, D, (int)pdl); break;
-    case 1: uq_launch(uq_fwht_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, D, (int)pdl); break;
-    default: uq_launch(uq_fwht_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const __half*)x, (__half*)out, rows, D, (int)pdl); break;
+    case 0: e = uq_launch(uq_fwht_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const float*)x, (float*)out, rows, D, (int)pdl); break;
+    case 1: e = uq_launch(uq_fwht_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, D, (int)pdl); break;
+    default: e = uq_launch(uq_fwht_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, (const __half*)x, (__half*)out, rows, D, (int)pdl); break;
   }
-  return cudaGetLastError();
+  return e;
 }
 
 // route: 0 by the size of the call, 4 the bulk kernel, 8 the per-row kernel (as the flags of uq_append_dispatch)
@@ -735,24 +736,25 @@ cudaError_t uq_append_nvfp4_dispatch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint
   if (!(D == 64 || D == 128 || D == 256) || PAGE <= 0 || HKV <= 0 || T < 0 || dtype < 0 || dtype > 2) return cudaErrorInvalidValue;
   if (!(k_ts > 0.f) || !(v_ts > 0.f) || (route != 0 && route != 4 && route != 8)) return cudaErrorInvalidValue;
   const long long warps = (long long)T * HKV * 2;
+  cudaError_t e = cudaSuccess;
   if (route == kRouteBulk || (route == 0 && warps >= kBulkMinRows)) {
     bool done = false;
     switch (dtype) {
-      case 0: done = bulk_nvfp4_launch<float>(kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, s); break;
-      case 1: done = bulk_nvfp4_launch<__nv_bfloat16>(kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, s); break;
-      default: done = bulk_nvfp4_launch<__half>(kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, s); break;
+      case 0: done = bulk_nvfp4_launch<float>(kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, s, e); break;
+      case 1: done = bulk_nvfp4_launch<__nv_bfloat16>(kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, s, e); break;
+      default: done = bulk_nvfp4_launch<__half>(kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, s, e); break;
     }
-    if (done) return cudaGetLastError();
+    if (done) return e;
     if (route == kRouteBulk) return cudaErrorInvalidValue;
   }
   const int blocks = (int)((warps + 3) / 4);
   const bool pdl = uq_pdl_on();
   switch (dtype) {
-    case 0: uq_launch(uq_append_nvfp4_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
-    case 1: uq_launch(uq_append_nvfp4_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
-    default: uq_launch(uq_append_nvfp4_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
+    case 0: e = uq_launch(uq_append_nvfp4_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
+    case 1: e = uq_launch(uq_append_nvfp4_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
+    default: e = uq_launch(uq_append_nvfp4_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, k_ts, v_ts, (int)pdl); break;
   }
-  return cudaGetLastError();
+  return e;
 }
 
 // dtype: 0 fp32, 1 bf16, 2 fp16.  value/vc/vs may be null (single-stream form).  flags: 1 rotate the keys, 2 'paper' rule with constant c,
@@ -769,24 +771,25 @@ cudaError_t uq_append_dispatch(uint8_t* kc, uint8_t* ks, uint8_t* vc, uint8_t* v
   flags &= 3;
   const int nstream = two ? 2 : 1;
   const long long warps = (long long)T * HKV * nstream;
+  cudaError_t e = cudaSuccess;
   // many rows: the bulk kernel (flags & 4 sends the call there whatever its size, flags & 8 keeps it here: the tests
   // compare the two on the same rows)
   if (route == kRouteBulk || (route == 0 && warps >= kBulkMinRows)) {
     bool done = false;
     switch (dtype) {
-      case 0: done = bulk_launch<float>(kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c, s); break;
-      case 1: done = bulk_launch<__nv_bfloat16>(kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c, s); break;
-      default: done = bulk_launch<__half>(kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c, s); break;
+      case 0: done = bulk_launch<float>(kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c, s, e); break;
+      case 1: done = bulk_launch<__nv_bfloat16>(kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c, s, e); break;
+      default: done = bulk_launch<__half>(kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c, s, e); break;
     }
-    if (done) return cudaGetLastError();
+    if (done) return e;
     if (route == kRouteBulk) return cudaErrorInvalidValue;   // asked for by name and not served (alignment, size)
   }
   const int blocks = (int)((warps + 3) / 4);
   const bool pdl = uq_pdl_on();
   switch (dtype) {
-    case 0: uq_launch(uq_append_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
-    case 1: uq_launch(uq_append_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
-    default: uq_launch(uq_append_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
+    case 0: e = uq_launch(uq_append_kernel<float>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const float*)key, (const float*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
+    case 1: e = uq_launch(uq_append_kernel<__nv_bfloat16>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
+    default: e = uq_launch(uq_append_kernel<__half>, dim3((unsigned)blocks), 128u, 0, s, pdl, kc, ks, vc, vs, (const __half*)key, (const __half*)value, slots, T, HKV, D, PAGE, nstream, flags, c, (int)pdl); break;
   }
-  return cudaGetLastError();
+  return e;
 }

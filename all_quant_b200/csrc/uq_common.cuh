@@ -47,7 +47,9 @@ inline cudaError_t uq_launch(void (*kern)(P...), dim3 grid, unsigned threads, si
   attr[0].val.programmaticStreamSerializationAllowed = dependent ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();   // the caller gets it as a value; left behind, it would be the next launch check's
+  return e;
 }
 
 // ---- what the host adds to UQParams for one launch -------------------------------------------------

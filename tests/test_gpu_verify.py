@@ -1,5 +1,6 @@
 """Parity of the CUDA verify/decode attention with the reference's known answers and with the CPU oracle,
 through the C ABI (all_quant_b200.uq_cuda -> libuq_b200.so).  Needs a B200."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -456,3 +457,34 @@ def test_the_switch_makes_every_launch_an_ordinary_one(cfg, programmatic):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", CAPTURED_CHAIN], cwd=root, env={**os.environ, "UQ_B200_CFG": cfg}, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and f"edges 6 programmatic {programmatic}" in r.stdout, r.stdout + r.stderr
+
+
+def test_a_launch_that_fails_leaves_no_error_for_the_next_one():
+    """Launches into a capture that has been invalidated (a synchronisation inside it) fail with the runtime's error; the next
+    ones, on a healthy stream, succeed: the failed launch's error is returned once and not left for a later launch check."""
+    B, K, HQ, HKV, D, PAGE, T = 2, 2, 8, 2, 64, 16, 40
+    kc, ks = (torch.zeros(8, HKV, PAGE, w, dtype=torch.uint8, device="cuda") for w in (D // 2, D // 32))
+    vc, vs = torch.zeros_like(kc), torch.zeros_like(ks)
+    key, slots = torch.randn(T, HKV, D, device="cuda").bfloat16(), torch.arange(T, device="cuda")
+    q, r, out = (torch.randn(B, K, HQ, D, device="cuda").bfloat16() for _ in range(3))
+    bt, sl = torch.arange(8, dtype=torch.int32, device="cuda").view(B, 4), torch.tensor([33, 7], dtype=torch.int32, device="cuda")
+    ws = torch.empty(uq_cuda.workspace_floats(B, K, HQ, HKV, D, 4), device="cuda")
+    o1, l1, m1 = torch.randn(2, B, K, HQ, D, device="cuda"), torch.randn(2, B, K, HQ, device="cuda"), torch.empty_like(q)
+    calls = [lambda: uq_cuda.uq_decode_cuda(q, kc, ks, vc, vs, bt, sl, nsplit=4, workspace=ws, out=out), lambda: uq_cuda.fwht(q, out=r),
+             lambda: uq_cuda.append_kv(kc, ks, vc, vs, key, key, slots, kernel="rows"), lambda: uq_cuda.append_kv(kc, ks, vc, vs, key, key, slots, kernel="bulk")]
+    after = calls + [lambda: uq_cuda.uq_merge(o1, l1, out=m1)]   # (the merge's launch check reads the runtime's last error)
+    for call in after:
+        call()
+    torch.cuda.synchronize()
+    cu, s, g = ctypes.CDLL("libcuda.so.1"), torch.cuda.Stream(), ctypes.c_void_p()
+    handle = ctypes.c_void_p(s.cuda_stream)
+    for failing in calls:
+        assert cu.cuStreamBeginCapture_v2(handle, 2) == 0
+        assert cu.cuStreamSynchronize(handle) != 0          # not allowed here: the capture is invalid from now on
+        with torch.cuda.stream(s), pytest.raises(RuntimeError):
+            failing()
+        assert cu.cuStreamEndCapture(handle, ctypes.byref(g)) != 0
+        for call in reversed(after):
+            call()
+    torch.cuda.synchronize()
+    assert uq_cuda.last_status() == (0, 0, 0, 0)
