@@ -344,7 +344,6 @@ int uqb_decode_partial_push_launch(const UQParams* p, const int32_t* pos_offset,
   push.rows_total = rows;
   push.world = world;
   push.seq = seq;
-  push.raise = 1;
   return (int)run(*p, pos_offset, nullptr, nullptr, reinterpret_cast<cudaStream_t>(stream), nullptr, &push);
 }
 

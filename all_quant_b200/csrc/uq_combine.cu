@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(128) uq_combine_kernel(const UQParams p, const
     }
   }
   }
-  if (kOut == 2 && push.raise) {
+  if (kOut == 2) {
     // the block that finishes last raises this rank's flag on every rank: each block's stores are fenced at system scope
     // before its ticket, and the last ticket holder fences again before the flags, so whoever sees a flag sees the partial
     __threadfence_system();

@@ -81,10 +81,9 @@ struct UQPeerPush {
   float* slot[kMaxPeers];          // this rank's slot in every rank's buffer, parity applied (slot[rank] is the local one)
   unsigned int* flag[kMaxPeers];   // this rank's flag word in every rank's buffer, parity applied
   unsigned int* counter;           // local word counting the combine's finished blocks (zero between calls)
-  size_t rows_total;               // rows of the whole call: the lse2 values follow rows_total * D floats of o
+  size_t rows_total;               // rows of the call: the lse2 values follow rows_total * D floats of o
   int world;
   unsigned int seq;
-  int raise;                       // 1: this launch is the call's last and raises the flags once its blocks are done
 };
 __host__ __device__ inline size_t uq_peer_slot_floats(size_t rows, int D) { return (rows * (size_t)(D + 1) + 3) / 4 * 4; }
 __host__ __device__ inline size_t uq_peer_data_bytes(int world, size_t slot_floats) { return ((size_t)2 * world * slot_floats * sizeof(float) + 255) / 256 * 256; }
