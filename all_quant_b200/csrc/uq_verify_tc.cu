@@ -129,6 +129,7 @@ __device__ unsigned long long g_tc_prof[5][8];
 #ifndef UQ_ABL
 #define UQ_ABL 0   // timing experiments only (results become wrong): 1 no exp2, 2 no P write, 4 no reference loads, 8 no score loads, 16 no work in the softmax's common tile, 32 no V decode, 64 no scale relay, 128 / 256 / 512 softmax / V / relay reduced to their waits and arrivals, 1024 no tensor instructions (commits only), 2048 no copies of the scale slices
 #endif
+constexpr bool kScaleCopies = !(UQ_ABL & 2048);
 constexpr int kKeys = 128;      // keys per tile = accumulator lanes
 // Thread layout: NSG softmax warpgroups (each owns NT / NSG query rows of every key), then K decode (4 warps), V decode (4),
 // producer, Q.K issue, P.V issue, one idle warp.  The roles are latency bound (one warp of a role per SM sub-partition issues
@@ -210,21 +211,18 @@ UQ_DEV void tc_commit(uint32_t bar) { asm volatile("tcgen05.commit.cta_group::1.
 // push out what every call comes back to (the queries, the page table, the partials the combine kernel reads, the kernel's
 // own instructions).
 #ifndef UQ_EVICT_FIRST
-#define UQ_EVICT_FIRST 1
+#define UQ_EVICT_FIRST 1   // 0: every copy with the normal policy
 #endif
-UQ_DEV uint64_t l2_evict_first_policy() {
+UQ_DEV uint64_t l2_policy() {
   uint64_t pol;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  if (UQ_EVICT_FIRST) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
   return pol;
 }
 // 2-D tiled TMA load: box (inner 0.., rows y..) of the tensor map into shared memory, bytes counted on `bar`.
 UQ_DEV void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar, uint64_t pol) {
-  if (UQ_EVICT_FIRST)
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "l"(pol) : "memory");
-  else
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "l"(pol) : "memory");
 }
 // contiguous bulk copy (scale pages)
 UQ_DEV void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t pol) {
@@ -878,7 +876,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
     const int spp_sh = __ffs(spp) - 1;
     UQ_PROF_DECL
     const uint32_t page_bytes_codes = (uint32_t)unit * C::kCodeRow, page_bytes_scales = (uint32_t)unit * C::kScaleB;
-    const uint64_t l2pol = l2_evict_first_policy();
+    const uint64_t l2pol = l2_policy();
     while (ok && next_seg(sg)) {
       if (!take()) continue;
       int off;
@@ -909,7 +907,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           for (int i0 = 0; i0 < kPieces; i0 += 32) {
             const int i = i0 + lane, key = i * (16 / C::kScaleB), u = key >> unit_sh;
             const int upid = __shfl_sync(0xffffffffu, pid, u & 31);
-            if (i < kPieces && u < vp) {
+            if (i < kPieces && u < vp && kScaleCopies) {
               const int in_page = spp_p2 ? (t * ppt + u) & (spp - 1) : (t * ppt + u) % spp;
               const size_t row = (size_t)(((long long)upid * p.HKV + sg.hk) * p.PAGE + in_page * unit + (key & (unit - 1)));
               cp_async16(dst + C::kOffKS + i * 16, p.ks + row * C::kScaleB);
@@ -919,7 +917,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           cp_async_arrive(bar_raw_full(stage));
           continue;
         }
-        if (lane == 0) mbar_expect_tx(bar_raw_full(stage), (uint32_t)vp * (page_bytes_codes + (kAsync ? 0u : page_bytes_scales)));
+        if (lane == 0) mbar_expect_tx(bar_raw_full(stage), (uint32_t)vp * (page_bytes_codes + (kAsync || !kScaleCopies ? 0u : page_bytes_scales)));
         __syncwarp();
         if (lane < vp) {
           // first cache row of this unit of (page, head); 64-bit: a cache may hold more than 2^31 / PAGE (page, head) slices
@@ -929,8 +927,8 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           // block-scaled: the K map unpacks (a page lands as PAGE x 128 bytes); the bytes counted on the barrier are the packed ones
           if (side & 1) tma_load_2d(dst + lane * (C::kBS ? 2 : 1) * page_bytes_codes, &map_kc, 0, (int)row0, fb, l2pol);
           if (side & 2) tma_load_2d(dst + C::kOffVC + lane * page_bytes_codes, &map_vc, 0, (int)row0, fb, l2pol);
-          if (!kAsync && (side & 4)) bulk_load(dst + C::kOffKS + lane * page_bytes_scales, p.ks + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
-          if (!kAsync && (side & 8)) bulk_load(dst + C::kOffVS + lane * page_bytes_scales, p.vs + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
+          if (!kAsync && kScaleCopies && (side & 4)) bulk_load(dst + C::kOffKS + lane * page_bytes_scales, p.ks + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
+          if (!kAsync && kScaleCopies && (side & 8)) bulk_load(dst + C::kOffVS + lane * page_bytes_scales, p.vs + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
         }
       }
     }
