@@ -29,7 +29,7 @@
 //                          key's codes and scale bytes are in registers.
 //   copy      2 warps      (K side / V side of every tile) TMA tensor copies of the code pages + bulk copies of the scale
 //                          pages into a ring of raw stages (3 at head_dim 128), mbarrier complete_tx.  No multicast.  Small pages
-//                          and head_dim 64 (dispatch_rows): a third warp brings the scale slices by per-lane asynchronous copies.
+//                          and head_dim 64 (async_unit): a third warp brings the scale slices by per-lane asynchronous copies.
 //   issue     1 thread     chosen by elect.sync: P.V of tile i, then Q.K of tile i + 2; tcgen05.commit to mbarriers; owns the
 //                          TMEM allocation.
 // Work is a flat list of tiles over all (sequence, kv head) items, cut into chunks of equal WEIGHT (an item counts its tiles
@@ -866,7 +866,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
   if (warp == kWarpProd || warp == kWarpProd + 2 || (kAsync && warp == kWarpProd + 3)) {
     // ================================================================= producer
     // Two warps, K side and V side: a lane per unit, a tensor copy of the codes and a bulk copy of the scale bytes.  A copy costs
-    // its issuing warp 250-350 cycles, one after the other; where that sets the pace (dispatch_rows) a third warp takes both
+    // its issuing warp 250-350 cycles, one after the other; where that sets the pace (async_unit) a third warp takes both
     // scale slices by ordinary asynchronous copies, 16 bytes per lane.
     const int side = warp == kWarpProd ? 5 : (!kAsync || warp == kWarpProd + 2 ? 10 : 0);   // bit 0 K codes, 1 V codes, 2 K scales, 3 V scales; 0: the third warp
     // a copy moves one unit: a whole page of up to 128 tokens, or a 128-token part of a larger page
@@ -1862,18 +1862,36 @@ int uq_verify_tc_splits(const UQParams& p, const UQLaunch& x) {
   return std::max(1, std::min(p.nsplit, span));
 }
 
+// Largest copy unit (tokens) with which the scale slices come by the third copy warp; 0 = never, kKeys = always.  Small units mean
+// many copies per tile, and their issue becomes the kernel's pace.  GPU time without / with it, in us (8 sequences of 8 K tokens;
+// head_dim 64: 16 of 4 K; head_dim 256: 4 of 16 K, half the heads; NVFP4 after the semicolon):
+//   head_dim 128, 16-token pages  16 rows 40.0 / 32.3, 32 rows 45.8 / 38.8, 64 rows 51.8 / 45.9; 43.5 / 35.5, 50.9 / 43.3, 56.3 / 47.5
+//                 32-token pages  16 rows 32.7 / 29.8, 32 rows 39.7 / 36.7, but 64 rows, where issue slots are short, 45.3 / 45.9; 35.6 / 32.8, 43.6 / 41.1
+//   head_dim 64 (tiles of half the bytes)
+//                 16-token pages  16 rows 42.7 / 34.0, 32 rows 50.1 / 40.0, 64 rows 57.1 / 49.2; 41.7 / 33.6
+//                 64 and more     16 rows 32.3 / 30.4 (64), 30.9 / 30.1 (128, 512), but 32 rows 39.4 / 39.8, 39.2 / 39.9, 39.2 / 39.9; 32 rows 38.9 / 39.5 (64)
+//   head_dim 256, 16-token pages  16 rows 39.3 / 38.9, 32 rows 43.4 / 42.4, but 64 rows 50.8 / 51.6; slower at every row count: 34.4 / 36.9, 40.6 / 41.8, 50.3 / 50.6
+//                 32-token pages  16 rows 37.9 / 37.5, 32 rows 42.4 / 42.0, 64 rows 50.8 / 51.2; 34.8 / 37.1, 40.7 / 42.1
+template <int D, int NT, int FMT>
+constexpr int async_unit() {
+  if (D == 256) return FMT == 1 || NT == 64 ? 0 : 32;
+  if (NT == 64) return 16;
+  return D == 64 && NT == 16 ? tc::kKeys : 32;
+}
+
+template <int D, int NT, int FMT>
+static cudaError_t dispatch_copy(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
+  constexpr int kUpTo = async_unit<D, NT, FMT>();
+  if constexpr (kUpTo == tc::kKeys) return tc::launch<D, NT, FMT, true>(p, x, s);
+  else if constexpr (kUpTo == 0) return tc::launch<D, NT, FMT, false>(p, x, s);
+  else return tc::copy_unit(p) <= kUpTo ? tc::launch<D, NT, FMT, true>(p, x, s) : tc::launch<D, NT, FMT, false>(p, x, s);
+}
+
 template <int D, int FMT>
 static cudaError_t dispatch_rows(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
-  // Small units mean many copies per tile, and their issue becomes the kernel's pace: the scale slices then come by a third copy
-  // warp.  GPU time without / with it (B=8, 8 K tokens; 16 sequences of 1 K .. 4 K for the one marked *): head_dim 128, 16-token pages
-  // 51.6 / 46.6 us at 64 rows, 40.9 / 34.3 at 16, NVFP4 52.9 / 45.1; 32-token pages 34.2 / 32.0 at 16 rows, but 45.4 / 46.7 at 64, where
-  // issue slots are short; 64-token pages level; head_dim 64, whose tiles are half the bytes: 16-token pages * 32.4 / 28.2, 32-token
-  // 35.8 / 32.8, 64-token 32.8 / 32.1.
-  const int unit = tc::copy_unit(p);
-  const bool some = unit <= 32 || D == 64, few = unit == 16;
-  if (x.rows <= 16) return some ? tc::launch<D, 16, FMT, true>(p, x, s) : tc::launch<D, 16, FMT, false>(p, x, s);
-  if (x.rows <= 32) return some ? tc::launch<D, 32, FMT, true>(p, x, s) : tc::launch<D, 32, FMT, false>(p, x, s);
-  return few ? tc::launch<D, 64, FMT, true>(p, x, s) : tc::launch<D, 64, FMT, false>(p, x, s);
+  if (x.rows <= 16) return dispatch_copy<D, 16, FMT>(p, x, s);
+  if (x.rows <= 32) return dispatch_copy<D, 32, FMT>(p, x, s);
+  return dispatch_copy<D, 64, FMT>(p, x, s);
 }
 
 cudaError_t uq_verify_tc_dispatch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
