@@ -1768,21 +1768,32 @@ int chunk_bound(const UQParams& p, const UQLaunch& x) {
   return x.ns_eff >= 2 ? (int)((max_tiles + x.ns_eff - 2) / (x.ns_eff - 1)) : 1;
 }
 
+// Multiprocessors of the current device (looked up once per device); 0 = not to be had.
+int current_sms() {
+  static std::atomic<int> cached[64];
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return 0;
+  sms = cached[dev].load(std::memory_order_relaxed);
+  if (sms <= 0) {
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) { cudaGetLastError(); return 0; }
+    cached[dev].store(sms, std::memory_order_relaxed);
+  }
+  return sms;
+}
+
 template <int D, int NT, int FMT, bool kAsync, bool kPick>
-cudaError_t launch_as(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
+cudaError_t launch_as(const UQParams& p, const UQLaunch& x, int sms, cudaStream_t s) {
   using C = Cfg<D, NT, FMT>;
   auto kern = uq_verify_tc_kernel<D, NT, FMT, kAsync, kPick>;
   static std::atomic<bool> ready[64];
-  static std::atomic<int> sm_counts[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (sms <= 0) return cudaErrorInitializationError;
   if (!ready[dev].load(std::memory_order_acquire)) {   // per device: the attribute belongs to the device's copy of the kernel
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
     if (e != cudaSuccess) { cudaGetLastError(); return e; }
-    int n = 0;
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    sm_counts[dev].store(n, std::memory_order_relaxed);
     ready[dev].store(true, std::memory_order_release);
   }
   Params prm;
@@ -1793,21 +1804,26 @@ cudaError_t launch_as(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   const int box_rows = copy_unit(p);
   prm.unit = box_rows;
   if (!cached_map(&mk, MapKey{p.kc, C::kCodeRow, box_rows, C::kBS ? 1 : 0}) || !cached_map(&mv, MapKey{p.vc, C::kCodeRow, box_rows, 0})) return cudaErrorInvalidValue;
-  const int sms = sm_counts[dev].load(std::memory_order_relaxed);
-  if (sms <= 0) return cudaErrorInitializationError;
   return uq_launch(kern, dim3(sms), cta_threads(NT), C::kSmem, s, x.pdl != 0, prm, mk, mv);
 }
 
-// The equal share of 148 CTAs is at most items x (longest table) / 148 tiles.  Where the bound is above a third of that - two or
-// three slots per item, with the default slot count from 150 items on - it is likely to bind for sequences of different length, and
-// the kernel looks for a smaller chunk (below eight tiles there is nothing to gain).  Elsewhere the code for that stays out: in every launch it cost up to 4 % of calls that
-// never use it (K=1, 8 sequences of 32 K tokens: 83.0 us, 85.8 with it).
+// Which launches look for a smaller chunk than the bound (pick_chunk): those with fewer than three (item, slot after the first) pairs
+// per SM, for bound and equal share both come from the table's width - the lengths are on the device - and it cancels.  With the default
+// slot count that is about 100 to 296 items (five slots down to two), and calls of one or two sequences, whose slots end at what an
+// item can span.  GPU time without / with the search, in us:
+//   tables as wide as the longest sequence   32 ragged sequences of 4 K .. 64 K tokens at K=8 445 / 420, of 1 K .. 32 K at K=1 178.8 / 170.2;
+//                                            equal lengths, nothing to find: 24 of 8 K at K=1 68.1 / 69.6, 32 of 8 K at K=8 136.2 / 137.7,
+//                                            one of 131 K on 4 heads at K=1 32.9 / 34.2
+//   tables for 131 072 tokens                one of 2 K 54.1 / 17.9, one of 16 K 58.2 / 25.1, two of 8 K at K=1 43.0 / 17.0, 32 of 2 K 840 / 63
+// The variant costs most of its calls 1 - 4 % where it finds nothing; other launches (8 sequences of 32 K at K=1: 83.0 / 85.8) go without,
+// although a table much wider than the sequences holds them back as well (8 of 2 K in one for 131 072: 117 / 29).
+// (Below eight tiles there is nothing to gain.)
 template <int D, int NT, int FMT, bool kAsync>
 cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
   const long long max_tiles = ((long long)p.max_pages * p.PAGE + kKeys - 1) / kKeys;
-  const int bound = chunk_bound(p, x);
-  const bool pick = x.ns_eff >= 2 && bound >= 8 && 3ll * 148 * bound > (long long)p.B * p.HKV * x.chunks * max_tiles;
-  return pick ? launch_as<D, NT, FMT, kAsync, true>(p, x, s) : launch_as<D, NT, FMT, kAsync, false>(p, x, s);
+  const int bound = chunk_bound(p, x), sms = current_sms();
+  const bool pick = x.ns_eff >= 2 && bound >= 8 && 3ll * sms * bound > (long long)p.B * p.HKV * x.chunks * max_tiles;
+  return pick ? launch_as<D, NT, FMT, kAsync, true>(p, x, sms, s) : launch_as<D, NT, FMT, kAsync, false>(p, x, sms, s);
 }
 
 }  // namespace tc
@@ -1850,14 +1866,8 @@ bool uq_verify_tc_serves(const UQParams& p, const UQLaunch& x) {
 // The flat list gives a CTA ceil(total / SMs) tiles and total >= Hkv x (tiles of the longest item), so an item spans at
 // most ceil(SMs / Hkv) + 1 CTAs; slots beyond that would only be marked empty by the kernel and skipped by the combine.
 int uq_verify_tc_splits(const UQParams& p, const UQLaunch& x) {
-  static std::atomic<int> cached[64];
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64) sms = cached[dev].load(std::memory_order_relaxed);
-  if (sms <= 0) {
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) { cudaGetLastError(); return p.nsplit; }
-    if (dev >= 0 && dev < 64) cached[dev].store(sms, std::memory_order_relaxed);
-  }
+  const int sms = tc::current_sms();
+  if (sms <= 0) return p.nsplit;
   const int span = (sms + p.HKV * x.chunks - 1) / (p.HKV * x.chunks) + 1;
   return std::max(1, std::min(p.nsplit, span));
 }

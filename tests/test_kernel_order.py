@@ -42,3 +42,9 @@ def test_indexes_of_read_only_loads_come_out_of_the_wait():
         assert body.count("uq_pdl_wait_index()") == 1 and "threadIdx" not in body, name
         wait = body.index("uq_pdl_wait_index()")
         assert not re.search(r"\b(key|value|slots|src|x)\s*\[|__ldg|\.load\(", body[:wait]), name
+
+
+def test_no_multiprocessor_count_is_written_down():
+    """The grid and the rules that compare with it ask the device for its count."""
+    for name in ("uq_verify_tc.cu", "uq_combine.cu", "uq_append.cu"):
+        assert not re.search(r"\b148\b", re.sub(r"//[^\n]*|asm volatile\([^;]*;", "", open(os.path.join(CSRC, name)).read())), name
