@@ -126,10 +126,6 @@ __device__ unsigned long long g_tc_prof[5][8];
 #ifndef UQ_NSG4_AT
 #define UQ_NSG4_AT 32
 #endif
-#ifndef UQ_ABL
-#define UQ_ABL 0   // timing experiments only (results become wrong): 1 no exp2, 2 no P write, 4 no reference loads, 8 no score loads, 16 no work in the softmax's common tile, 32 no V decode, 64 no scale relay, 128 / 256 / 512 softmax / V / relay reduced to their waits and arrivals, 1024 no tensor instructions (commits only), 2048 no copies of the scale slices
-#endif
-constexpr bool kScaleCopies = !(UQ_ABL & 2048);
 constexpr int kKeys = 128;      // keys per tile = accumulator lanes
 // Thread layout: NSG softmax warpgroups (each owns NT / NSG query rows of every key), then K decode (4 warps), V decode (4),
 // producer, Q.K issue, P.V issue, one idle warp.  The roles are latency bound (one warp of a role per SM sub-partition issues
@@ -907,7 +903,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           for (int i0 = 0; i0 < kPieces; i0 += 32) {
             const int i = i0 + lane, key = i * (16 / C::kScaleB), u = key >> unit_sh;
             const int upid = __shfl_sync(0xffffffffu, pid, u & 31);
-            if (i < kPieces && u < vp && kScaleCopies) {
+            if (i < kPieces && u < vp) {
               const int in_page = spp_p2 ? (t * ppt + u) & (spp - 1) : (t * ppt + u) % spp;
               const size_t row = (size_t)(((long long)upid * p.HKV + sg.hk) * p.PAGE + in_page * unit + (key & (unit - 1)));
               cp_async16(dst + C::kOffKS + i * 16, p.ks + row * C::kScaleB);
@@ -917,7 +913,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           cp_async_arrive(bar_raw_full(stage));
           continue;
         }
-        if (lane == 0) mbar_expect_tx(bar_raw_full(stage), (uint32_t)vp * (page_bytes_codes + (kAsync || !kScaleCopies ? 0u : page_bytes_scales)));
+        if (lane == 0) mbar_expect_tx(bar_raw_full(stage), (uint32_t)vp * (page_bytes_codes + (kAsync ? 0u : page_bytes_scales)));
         __syncwarp();
         if (lane < vp) {
           // first cache row of this unit of (page, head); 64-bit: a cache may hold more than 2^31 / PAGE (page, head) slices
@@ -927,8 +923,8 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           // block-scaled: the K map unpacks (a page lands as PAGE x 128 bytes); the bytes counted on the barrier are the packed ones
           if (side & 1) tma_load_2d(dst + lane * (C::kBS ? 2 : 1) * page_bytes_codes, &map_kc, 0, (int)row0, fb, l2pol);
           if (side & 2) tma_load_2d(dst + C::kOffVC + lane * page_bytes_codes, &map_vc, 0, (int)row0, fb, l2pol);
-          if (!kAsync && kScaleCopies && (side & 4)) bulk_load(dst + C::kOffKS + lane * page_bytes_scales, p.ks + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
-          if (!kAsync && kScaleCopies && (side & 8)) bulk_load(dst + C::kOffVS + lane * page_bytes_scales, p.vs + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
+          if (!kAsync && (side & 4)) bulk_load(dst + C::kOffKS + lane * page_bytes_scales, p.ks + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
+          if (!kAsync && (side & 8)) bulk_load(dst + C::kOffVS + lane * page_bytes_scales, p.vs + (size_t)row0 * C::kScaleB, page_bytes_scales, fb, l2pol);
         }
       }
     }
@@ -973,10 +969,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           tc_fence_after();
           UQ_TRACE(5, c)
           const uint32_t d = tmem + C::cS + buf * C::kSCols, a = tmem + C::cK + buf * C::kKCols;
-          if (UQ_ABL & 1024) {
-            tc_commit(bar(bSfull + buf));
-            if (C::kBS) tc_commit(bar_raw_empty(c % kRawStages));
-          } else if constexpr (C::kBS) {
+          if constexpr (C::kBS) {
             // A = the unpacked K codes of the tile's raw stage (K-major, 128-byte rows), B = the leading and the remainder tile of Q
             const int stage = c % kRawStages;
             const uint64_t a_desc = smem_desc(sm_a + C::oRaw + stage * C::kRawStage, 16, 1024);
@@ -1015,7 +1008,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           // (a P^T slot inside a shared buffer starts (slot % kPPer) * NT rows = that many * 2 bytes into every key's row)
           const uint64_t va = v_desc + (uint64_t)(vb * (C::kVTile >> 4)), pa = p_desc + (uint64_t)((buf / C::kPPer) * (C::kPTile >> 4) + (buf % C::kPPer) * (NT * 2 >> 4));
 #pragma unroll
-          for (int db = 0; db < ((UQ_ABL & 1024) ? 0 : C::kDB); db++) {
+          for (int db = 0; db < C::kDB; db++) {
 #pragma unroll
             for (int kk = 0; kk < kKeys / 16; kk++)
               mma_ss(tmem + C::cO + db * NT, va + (uint64_t)((db * 2 * C::kVHalf + kk * 2048) >> 4), pa + (uint64_t)(kk * (2048 >> 4)), idesc_pv, (i == 0 && kk == 0) ? 0u : 1u);
@@ -1049,7 +1042,6 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         if (ok && cnt >= kSB) ok = wait(bar(bSfull + buf), sp.phase ^ 1u, 44 + buf, cnt UQ_PROF_SITE(1));   // S^T of the tile that used this buffer is done: the A operand is free
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if ((UQ_ABL & 512) && cnt) { warp_arrive(bar(bKfull + buf)); warp_arrive(bar_raw_empty(stage)); continue; }
         tc_fence_after();
         if (kk == 0) { UQ_TRACE(1, cnt) }
         UQ_PROF_T0
@@ -1066,11 +1058,9 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         if constexpr (C::kBS) {
           // block-scaled: nothing to decode.  The contraction wants the scale bytes of key 32 j + l (one 32-bit word: byte b =
           // channels 32 b ..) in column j of lane l of every 32-lane quarter: each warp writes its quarter.
-          if (!(UQ_ABL & 64) || cnt == 0) {
-            const uint32_t* ksw = reinterpret_cast<const uint32_t*>(raw + C::kOffKS);
-            const uint32_t w4[4] = {ksw[lane], ksw[32 + lane], ksw[64 + lane], ksw[96 + lane]};
-            tmem_st4(lane_addr + C::cK + buf * C::kKCols, w4);
-          }
+          const uint32_t* ksw = reinterpret_cast<const uint32_t*>(raw + C::kOffKS);
+          const uint32_t w4[4] = {ksw[lane], ksw[32 + lane], ksw[64 + lane], ksw[96 + lane]};
+          tmem_st4(lane_addr + C::cK + buf * C::kKCols, w4);
         } else {
         // the code row of this key: chunk g (16 bytes = group g) sits at chunk g ^ ((key / rows per 128 B) mod chunks) (TMA swizzle)
         const uint8_t* krow = raw + kk * C::kCodeRow;
@@ -1126,7 +1116,6 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         if (ok && cnt >= kVB) ok = wait(bar(bVdone + buf), vp.phase ^ 1u, 54 + buf, cnt UQ_PROF_SITE(1));   // O^T += of the tile that used this buffer is done
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if ((UQ_ABL & 256) && cnt) { warp_arrive(bar(bVfull + buf)); warp_arrive(bar_raw_empty(stage)); continue; }
         if (vw == 0 && lane == 0) { UQ_TRACE(3, cnt) }
         UQ_PROF_T0
         const uint8_t* raw = sm + C::oRaw + stage * C::kRawStage + C::kOffVC;
@@ -1147,7 +1136,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           for (int g = 0; g < kGPT; g++) vs2[g] = *reinterpret_cast<const uint16_t*>(vsc + 2 * (gfirst + g));
         }
 #pragma unroll
-        for (int gb = 0; gb < ((UQ_ABL & 32) && cnt ? 0 : kGPT); gb += 4) {
+        for (int gb = 0; gb < kGPT; gb += 4) {
           constexpr int GN = kGPT < 4 ? kGPT : 4;
           const int g0 = gfirst + gb;
           uint4 c4[GN];
@@ -1177,7 +1166,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         UQ_PROF_T1(2)
         fence_async_smem();
         warp_arrive(bar(bVfull + buf));
-        if (!UQ_EARLY || ((UQ_ABL & 32) && cnt)) warp_arrive(bar_raw_empty(stage));
+        if (!UQ_EARLY) warp_arrive(bar_raw_empty(stage));
         if (vw == 0 && lane == 0) { UQ_TRACE(4, cnt) }
         UQ_PROF_T1(3)
       }
@@ -1396,7 +1385,6 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
             bool r = wait(bar(bSfull + buf), sph, 62 + buf, cnt UQ_PROF_SITE(0));
             r = __all_sync(0xffffffffu, r);
             if (!r) { ok = false; break; }
-            if (UQ_ABL & 128) { warp_arrive(bar(bPfull + buf)); if (++buf == kSB) { buf = 0; sph ^= 1u; } continue; }
             tc_fence_after();
             if (st == 0) { UQ_TRACE(9, cnt) }
             float pv[HW];
@@ -1465,9 +1453,9 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           float xm = kNegBig;
 #pragma unroll
           for (int i = 0; i < HW; i++) {
-            float xv = fmaf(pv[i], ck, (UQ_ABL & 4) ? -1.0f : -mrow[r0 + i]);
+            float xv = fmaf(pv[i], ck, -mrow[r0 + i]);
             xm = fmaxf(xm, xv);
-            pv[i] = (UQ_ABL & 1) ? xv * 0.001f : fast_exp2(xv);
+            pv[i] = fast_exp2(xv);
           }
           return xm;
         };
@@ -1491,11 +1479,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
             for (int i = 0; i < HW; i++) pv[i] = ((vmask >> i) & 1u) ? pv[i] : -INFINITY;
           }
         };
-        if (!(UQ_ABL & (8 | 16)) || cnt == c0) load_masked();
-        else {
-#pragma unroll
-          for (int i = 0; i < HW; i++) pv[i] = 0.5f;
-        }
+        load_masked();
         if (st == 0) { UQ_TRACE(10, cnt) }
         UQ_PROF_TB(2)
         const int rbyte = (int)wr[4 + mcur];
@@ -1503,7 +1487,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
         const bool agree = careful && !first;      // later tiles agree on a move only on the careful path
         const bool lean = !careful && !first && !need_mask;
         float xm = kNegBig;
-        if (first || (lean && (UQ_ABL & 16))) {
+        if (first) {
         } else if (lean) {
           // the common tile: 2^(s * ck - m) as 2^-(s * (-ck) + m), two rows per fused multiply-add
           const float4* m4 = reinterpret_cast<const float4*>(mref + mcur * NT + r0);
@@ -1518,7 +1502,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           }
         } else xm = probabilities(mref + mcur * NT);
         UQ_PROF_TB(3)
-        if (!first && !(UQ_ABL & 2) && !((UQ_ABL & 16) && lean)) write_p(rbyte);
+        if (!first) write_p(rbyte);
         if (st == 0) { UQ_TRACE(11, cnt) }
         UQ_PROF_TB(4)
         // ---- did any score leave the window of its row's reference, or any key's V scale exceed the segment's reference?
@@ -1532,7 +1516,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           if (!ok) break;
         } else if (!first) {
           // quick path: what this tile wrote may have overflowed; mark the segment for the second pass and carry on
-          if (!UQ_ABL && grew && lane == 0) { atomicOr(&redo[ord >> 5], 1u << (ord & 31)); redo[kRedoWords] = 1u; }
+          if (grew && lane == 0) { atomicOr(&redo[ord >> 5], 1u << (ord & 31)); redo[kRedoWords] = 1u; }
         }
         if (first || (agree && *reinterpret_cast<volatile int*>(&vote[vslot]))) {
           UQ_PROF_COUNT(6)
@@ -1592,10 +1576,8 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           write_p((int)wr[4 + mcur]);
         }
         UQ_PROF_TA2
-        if (!((UQ_ABL & 16) && lean)) {
 #pragma unroll
-          for (int i = 0; i < HW; i += 2) add_f32x2(l[i], l[i + 1], pv[i], pv[i + 1]);
-        }
+        for (int i = 0; i < HW; i += 2) add_f32x2(l[i], l[i + 1], pv[i], pv[i + 1]);
         tc_fence_before();
         fence_async_smem();
         warp_arrive(bar(bPfull + buf));   // P^T is written; it also tells the Q.K issuer that this slot's S^T is consumed
@@ -1652,7 +1634,7 @@ uq_verify_tc_kernel(const __grid_constant__ Params prm, const __grid_constant__ 
           }
         }
         // quick path: the segment's result is garbage then; the second pass computes it again on the careful path
-        if (!UQ_ABL && !careful && __any_sync(0xffffffffu, bad) && lane == 0) { atomicOr(&redo[ord >> 5], 1u << (ord & 31)); redo[kRedoWords] = 1u; }
+        if (!careful && __any_sync(0xffffffffu, bad) && lane == 0) { atomicOr(&redo[ord >> 5], 1u << (ord & 31)); redo[kRedoWords] = 1u; }
         if (st < rows) { const float lr = (lsum[st] + lsum[NT + st]) + (lsum[2 * NT + st] + lsum[3 * NT + st]); ml[st] = lr > 0.f ? mr[st] + log2f(lr) : -INFINITY; }
       }
       tc_fence_before();
