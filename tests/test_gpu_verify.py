@@ -169,17 +169,20 @@ def test_scale_slices_of_small_copies_come_by_a_third_warp(D, PAGE, rows, fmt):
     npg = -(-int(sl.max()) // PAGE)
     shape = lambda row: (B * npg, HKV, PAGE, row)
     kc, vc = (rng.integers(0, 256, shape(D // 2), dtype=np.uint8) for _ in range(2))
-    lo, hi, per = (125, 130, 32) if fmt == 0 else (0x30, 0x40, 16)
-    ks, vs = (rng.integers(lo, hi, shape(D // per)).astype(np.uint8) for _ in range(2))
+    # Scales and queries for which every key counts: with the 16 bytes of a neighbour in the place of any one piece, K or V, some row of
+    # the oracle's answer moves by more than 1.5 % of its largest entry (98 % of the pieces or more, by format and head size).
+    per, kr, vr, qs = (32, (124, 128), (125, 129), 0.4) if fmt == 0 else (16, (0x28, 0x48), (0x28, 0x48), 0.3)
+    ks, vs = (rng.integers(*r, shape(D // per)).astype(np.uint8) for r in (kr, vr))
     bt = rng.permutation(B * npg).astype(np.int32).reshape(B, npg)
-    qb = O.bf16_bits(0.3 * rng.standard_normal((B, K, HKV * G, D)).astype(np.float32))
+    qb = O.bf16_bits(qs * rng.standard_normal((B, K, HKV * G, D)).astype(np.float32))
     ref = O.reference(qb, kc, ks, vc, vs, bt, sl) if fmt == 0 else O.reference_nvfp4(qb, kc, ks, vc, vs, bt, sl, 0.5, 0.5)
     out = uq_cuda.uq_decode_cuda(dev(qb.view(np.int16), torch.bfloat16), *(dev(a) for a in (kc, ks, vc, vs, bt, sl)),
                                  **(dict(fmt=1, k_ts=0.5, v_ts=0.5) if fmt else {}))
     assert uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
-    # (a sequence of one key returns that key's value, up to 24 here, rounded to bf16 - half an ulp is 2^-9 of it - while the rule's mean
-    # bound is absolute and meant for outputs of O(1): compared relative to the largest)
-    mx = np.abs(ref).max()
+    # row by row relative to the row's largest: a sequence of one key returns values up to 24, one of 637 keys small sums, and the
+    # rounding of bf16 (2^-9 of an entry) is far below the rule's 1 % in each
+    mx = np.abs(ref).max(-1, keepdims=True)
+    mx[mx == 0] = 1
     check_close(out.float().cpu().numpy() / mx, ref / mx, f"PAGE={PAGE}")
 
 
