@@ -354,43 +354,71 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_call_is_unaffected(monkey
         assert uq_cuda.last_status() == (0, 0, 0, 0) and uq_cuda.last_path() == 2
         check_close(out.float().cpu().numpy(), c.ref, "call after a wait that ran out")
 
-@pytest.mark.parametrize("rotate", [False, True])
-def test_a_chain_of_calls_needs_no_synchronisation(rotate):
-    """Every kernel is set up while the one before it on the stream still runs and waits for it before it touches memory: steps
-    that write the cache, the queries and the scratch the neighbouring steps read give the bits of the same steps run apart."""
-    B, K, HQ, HKV, D, PAGE, ctx, steps = 4, 2, 16, 4, 128, 64, 900, 12
+
+@pytest.mark.parametrize("mode", ["together", "graph"])
+@pytest.mark.parametrize("chain,fmt,ctx,K", [("append verify", 0, 900, 2), ("append verify", 1, 900, 2), ("append rotate verify", 0, 900, 2), ("append append verify", 0, 900, 2),
+                                             ("verify verify", 0, 900, 8), ("append verify", 0, 9000, 1), ("append rotate verify", 0, 300, 16)])
+def test_a_chain_of_calls_needs_no_synchronisation(chain, fmt, ctx, K, mode):
+    """Every kernel is set up while the one before it on the stream still runs and waits for it before it touches memory.  Calls that
+    write what the next one reads - cache, queries, scratch - follow each other with nothing of torch's in between, eagerly and replayed
+    from a graph, and give the bits of the same calls run apart.  Every step rewrites the whole cache with other tokens (from 9000 per
+    sequence on in several thousand blocks of the bulk kernel), so that anything read too early is another step's."""
+    B, HQ, HKV, D, PAGE, steps = 4, 16, 4, 128, 64, 4 if ctx > 4000 else 10
     g = torch.Generator(device="cuda").manual_seed(5)
     npg = -(-ctx // PAGE)
     bt = torch.randperm(B * npg, generator=g, device="cuda").to(torch.int32).view(B, npg)
-    key = torch.randn(B * ctx, HKV, D, generator=g, device="cuda").bfloat16()
-    value = torch.randn(B * ctx, HKV, D, generator=g, device="cuda").bfloat16()
     pos = torch.arange(ctx, device="cuda").repeat(B)
     slots = bt.long().repeat_interleave(ctx, 0)[torch.arange(B * ctx, device="cuda"), pos // PAGE] * PAGE + pos % PAGE
-    q0 = torch.randn(steps, B, K, HQ, D, generator=g, device="cuda").bfloat16()
+    sl = torch.full((B,), ctx, dtype=torch.int32, device="cuda")
+    key, value = ([torch.randn(B * ctx, HKV, D, generator=g, device="cuda").bfloat16() for _ in range(steps)] for _ in range(2))
+    q = [torch.randn(B, K, HQ, D, generator=g, device="cuda").bfloat16() for _ in range(steps)]
+    cache = [torch.zeros(B * npg, HKV, PAGE, w, dtype=torch.uint8, device="cuda") for w in (D // 2, D // (16 if fmt else 32)) * 2]
     ws = torch.empty(uq_cuda.workspace_floats(B, K, HQ, HKV, D, 8), device="cuda")
+    rot, outs = torch.empty_like(q[0]), [torch.empty_like(q[0]) for _ in range(2 * steps)]
+    ts = dict(fmt=1, k_ts=0.01, v_ts=0.01) if fmt else {}
 
-    def run(sync):
-        kc = torch.zeros(B * npg, HKV, PAGE, D // 2, dtype=torch.uint8, device="cuda")
-        ks = torch.zeros(B * npg, HKV, PAGE, D // 32, dtype=torch.uint8, device="cuda")
-        vc, vs = torch.zeros_like(kc), torch.zeros_like(ks)
-        q, out, outs = torch.empty_like(q0[0]), torch.empty_like(q0[0]), []
-        uq_cuda.append_kv(kc, ks, vc, vs, key, value, slots, rotate_k=rotate)
+    def append(k, v, rotate):
+        if fmt:
+            uq_cuda.append_kv_nvfp4(*cache, k, v, slots, 0.01, 0.01)
+        else:
+            uq_cuda.append_kv(*cache, k, v, slots, rotate_k=rotate)
+
+    def run(after):
         for s in range(steps):
-            new = torch.arange(s, B * ctx, steps, device="cuda")   # other tokens in every step, overwritten with a shifted input
-            q.copy_(q0[s])
-            for call in (lambda: uq_cuda.append_kv(kc, ks, vc, vs, key[(new + s + 1) % (B * ctx)], value[new], slots[new], rotate_k=rotate),
-                         lambda: q.copy_(uq_cuda.fwht(q)),
-                         lambda: uq_cuda.uq_decode_cuda(q, kc, ks, vc, vs, bt, torch.full((B,), ctx, dtype=torch.int32, device="cuda"), nsplit=8, workspace=ws, out=out),
-                         lambda: outs.append(out.clone())):
-                call()
-                if sync:
-                    torch.cuda.synchronize()
-        torch.cuda.synchronize()
-        return torch.stack(outs), kc, vs
+            n, last = 0, q[s]
+            for what in chain.split():
+                if what == "append":
+                    append(key[(s + n) % steps], value[s], "rotate" in chain)
+                elif what == "rotate":
+                    last = uq_cuda.fwht(q[s], out=rot)
+                else:
+                    uq_cuda.uq_decode_cuda(last, *cache, bt, sl, nsplit=8, workspace=ws, out=outs[2 * s + n % 2], **ts)
+                    last = q[(s + 1) % steps]
+                n += 1
+                after()
 
-    for a, b in zip(run(False), run(True)):
+    def result(how):
+        for t in (*cache, *outs, rot, ws):
+            t.zero_()
+        if "append" not in chain:
+            append(key[0], value[0], False)
+        torch.cuda.synchronize()
+        how()
+        torch.cuda.synchronize()
+        return [t.clone() for t in (*outs, *cache)]
+
+    def graph():
+        graphs = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graphs):
+            run(lambda: None)
+        graphs.replay()
+
+    apart = result(lambda: run(torch.cuda.synchronize))
+    assert uq_cuda.last_path() == 2
+    for a, b in zip(apart, result(graph if mode == "graph" else lambda: run(lambda: None))):
         assert torch.equal(a, b)
-    assert uq_cuda.last_status() == (0, 0, 0, 0)
+    assert any(bool(t.any()) for t in apart[:2]) and uq_cuda.last_status() == (0, 0, 0, 0)
+
 
 @pytest.mark.parametrize("nsplit", [2, 3])
 @pytest.mark.parametrize("B,HKV,long_ones,longest,width", [(40, 4, 3, 3000, 3000), (40, 4, 3, 3000, 40000), (150, 1, 1, 9000, 9000), (33, 8, 33, 1500, 1500), (3, 1, 3, 20000, 20000)])
