@@ -40,13 +40,13 @@
 // Every wait is bounded (about one second): on expiry the thread records the barrier in the status record, raises the CTA's
 // abort flag and every role drains to the common exit, which frees TMEM.
 //
-// Where the time goes (headline shape, K=8, B200): the call is bound neither by HBM (the same call on an L2-resident cache is
-// 3 % faster), nor by the tensor pipe (without its instructions: 2 % faster), but by the roles' serial chains: with every
-// role reduced to its waits and arrivals and the tensor instructions left out, the copy ring and the hand-shakes alone take
-// 91 us against 122 for the whole call.  Per CTA the time is 0.85 us per tile (1 660 cycles; the four V-decode warps are the
-// longest role: 1 210 cycles of decode, 450 between tiles) plus about 25 us that do not depend on the context: set-up,
-// the first segment's query conversion and first tile (which fixes the references), the epilogue, and the spread of the
-// CTAs' finishing times.
+// Where the time goes (8 sequences of 32 K tokens, head_dim 128, 64-token pages, GPU time from a graph at 1965 MHz): 115.6 us at 64 rows, 83.0 at 8, against
+// 44 for the bytes at the copy rate.  Not the tensor pipe (without its instructions 115.1 / 78.3), but the roles' serial chains:
+// with every role reduced to its waits and arrivals and the tensor instructions left out, the copy ring and the hand-shakes
+// alone take 77 / 64 us, 71 / 54 when the scale slices' copies are left out too; the softmax's arithmetic adds 16 / 5, the V decode's 16 / 9.
+// Over the context length that is 0.84 us per tile and CTA (K=1: 0.64) plus 22 us (12.5) that do not depend on it: set-up, the first
+// segment's query conversion and first tile (which fixes the references), the epilogue, the combine, and the spread of the CTAs'
+// finishing times.  Under a load of seconds the K=8 call runs at the power limit: 130 us at 1755 MHz (83 -> 84.5 at K=1, 1935 MHz).
 #include <cuda.h>
 
 #include <algorithm>
@@ -127,9 +127,9 @@ __device__ unsigned long long g_tc_prof[5][8];
 #define UQ_NSG4_AT 32
 #endif
 constexpr int kKeys = 128;      // keys per tile = accumulator lanes
-// Thread layout: NSG softmax warpgroups (each owns NT / NSG query rows of every key), then K decode (4 warps), V decode (4),
-// producer, Q.K issue, P.V issue, one idle warp.  The roles are latency bound (one warp of a role per SM sub-partition issues
-// about once per 10 cycles), so the softmax, the longest role at 64 rows, is spread over four warpgroups.
+// Thread layout: NSG softmax warpgroups (each owns NT / NSG query rows of every key), then K decode or relay (4 warps), V decode (4 or 8),
+// copy K side, issue, copy V side, copy scale slices (idle without kAsync).  The roles are latency bound (one warp of a role per SM
+// sub-partition issues about once per 10 cycles), so the softmax, the longest role at 64 rows, is spread over four warpgroups.
 __host__ __device__ constexpr int softmax_groups(int NT) { return NT >= UQ_NSG4_AT ? 4 : 2; }
 // With fewer than 64 rows the V decode is the longest role and the CTA has warps to spare: eight V warps, each thread
 // half of its key's scale groups; with 64 rows the softmax is, and issue slots are what it lacks: four V warps.
@@ -1855,15 +1855,20 @@ int uq_verify_tc_splits(const UQParams& p, const UQLaunch& x) {
 }
 
 // Largest copy unit (tokens) with which the scale slices come by the third copy warp; 0 = never, kKeys = always.  Small units mean
-// many copies per tile, and their issue becomes the kernel's pace.  GPU time without / with it, in us (8 sequences of 8 K tokens;
-// head_dim 64: 16 of 4 K; head_dim 256: 4 of 16 K, half the heads; NVFP4 after the semicolon):
-//   head_dim 128, 16-token pages  16 rows 40.0 / 32.3, 32 rows 45.8 / 38.8, 64 rows 51.8 / 45.9; 43.5 / 35.5, 50.9 / 43.3, 56.3 / 47.5
-//                 32-token pages  16 rows 32.7 / 29.8, 32 rows 39.7 / 36.7, but 64 rows, where issue slots are short, 45.3 / 45.9; 35.6 / 32.8, 43.6 / 41.1
-//   head_dim 64 (tiles of half the bytes)
-//                 16-token pages  16 rows 42.7 / 34.0, 32 rows 50.1 / 40.0, 64 rows 57.1 / 49.2; 41.7 / 33.6
-//                 64 and more     16 rows 32.3 / 30.4 (64), 30.9 / 30.1 (128, 512), but 32 rows 39.4 / 39.8, 39.2 / 39.9, 39.2 / 39.9; 32 rows 38.9 / 39.5 (64)
-//   head_dim 256, 16-token pages  16 rows 39.3 / 38.9, 32 rows 43.4 / 42.4, but 64 rows 50.8 / 51.6; slower at every row count: 34.4 / 36.9, 40.6 / 41.8, 50.3 / 50.6
-//                 32-token pages  16 rows 37.9 / 37.5, 32 rows 42.4 / 42.0, 64 rows 50.8 / 51.2; 34.8 / 37.1, 40.7 / 42.1
+// many copies per tile, and their issue becomes the kernel's pace.  GPU time without / with it in us, at up to 16 rows, 32 rows, 64 rows
+// (8 sequences of 8 K tokens; head_dim 64: 16 of 4 K; head_dim 256: 4 of 16 K on half the heads):
+//                               UltraQuant                              NVFP4
+//   head_dim 64,   16-token     42.7 / 34.0  50.1 / 40.0  57.1 / 49.2   41.7 / 33.6  49.4 / 40.6  56.8 / 48.8   (tiles of half the bytes)
+//                  32-token     35.3 / 31.0  42.4 / 39.8  49.8 / 49.1   34.0 / 30.5  41.6 / 39.3  49.5 / 48.7
+//                  64-token     32.3 / 30.4  39.4 / 39.8  48.8 / 49.2   30.9 / 29.8  38.9 / 39.5
+//                  128-token    30.9 / 30.1  39.2 / 39.9                29.6 / 29.6  38.7 / 39.5                (512-token pages the same)
+//   head_dim 128,  16-token     40.0 / 32.3  45.8 / 38.8  51.8 / 45.9   43.5 / 35.5  50.9 / 43.3  56.3 / 47.5
+//                  32-token     32.7 / 29.8  39.7 / 36.7  45.3 / 45.9   35.6 / 32.8  43.6 / 41.1  48.9 / 46.2
+//                  64-token     29.8 / 29.6
+//   head_dim 256,  16-token     39.3 / 38.9  43.4 / 42.4  50.8 / 51.6   34.4 / 36.9  40.6 / 41.8  50.3 / 50.6
+//                  32-token     37.9 / 37.5  42.4 / 42.0  50.8 / 51.2   34.8 / 37.1  40.7 / 42.1
+// At 64 rows issue slots are short: 16-token units only, although 32-token ones would gain at head_dim 64 and for NVFP4.  The copies carry no
+// cache hint: with the evict-first policy of the others they were level or up to 0.3 us slower.
 template <int D, int NT, int FMT>
 constexpr int async_unit() {
   if (D == 256) return FMT == 1 || NT == 64 ? 0 : 32;
