@@ -90,9 +90,9 @@ def peaks():
         return 6650.0, "fallback"
 
 
-# DRAM traffic of one launch of the attention kernel from the ncu capture summarised in the named file (dram__bytes_read.sum +
+# DRAM traffic of one launch of the attention kernel from the ncu capture named here (dram__bytes_read.sum +
 # dram__bytes_write.sum of a half-size headline call, whose algorithmic bytes are given beside it); None = no capture on record
-TRAFFIC_PROFILE = {"source": "profiles/uq_verify_tc_kernel_ctx16384_K8_ncu_full.md", "dram_bytes": 145.7e6 + 12.5e6, "algorithmic_bytes": 142606336}
+TRAFFIC_PROFILE = {"source": "ncu capture of the attention kernel: headline shape at 16384 tokens, K=8", "dram_bytes": 145.7e6 + 12.5e6, "algorithmic_bytes": 142606336}
 
 
 def kv_bytes(cfg, seq_lens):
