@@ -44,6 +44,12 @@ def test_indexes_of_read_only_loads_come_out_of_the_wait():
         assert not re.search(r"\b(key|value|slots|src|x)\s*\[|__ldg|\.load\(", body[:wait]), name
 
 
+def test_appends_release_their_successors_after_their_own_wait():
+    """Before it, a waiting kernel would let the next one in, and that one the next: a pile of waiting grids in the working one's way."""
+    for name, body in kernels("uq_append.cu").items():
+        assert body.count("uq_pdl_release()") == 1 and body.index("uq_pdl_release()") > body.index("uq_pdl_wait_index()"), name
+
+
 def test_no_multiprocessor_count_is_written_down():
     """The grid and the rules that compare with it ask the device for its count."""
     for name in ("uq_verify_tc.cu", "uq_combine.cu", "uq_append.cu"):
