@@ -1792,20 +1792,20 @@ cudaError_t launch_as(const UQParams& p, const UQLaunch& x, int sms, cudaStream_
 // Which launches look for a smaller chunk than the bound (pick_chunk): those with fewer than three (item, slot after the first) pairs
 // per SM, for bound and equal share both come from the table's width - the lengths are on the device - and it cancels.  With the default
 // slot count that is about 100 to 296 items (five slots down to two), and calls of one or two sequences, whose slots end at what an
-// item can span.  GPU time without / with the search, in us:
+// item can span.  GPU time without / with the search, in us (both without the third copy warp, which searching launches of up to 32 rows
+// at head_dim 128 take besides, see async_unit):
 //   tables as wide as the longest sequence   32 ragged sequences of 4 K .. 64 K tokens at K=8 445 / 420, of 1 K .. 32 K at K=1 178.8 / 170.2;
 //                                            equal lengths, nothing to find: 24 of 8 K at K=1 68.1 / 69.6, 32 of 8 K at K=8 136.2 / 137.7,
 //                                            one of 131 K on 4 heads at K=1 32.9 / 34.2
 //   tables for 131 072 tokens                one of 2 K 54.1 / 17.9, one of 16 K 58.2 / 25.1, two of 8 K at K=1 43.0 / 17.0, 32 of 2 K 840 / 63
-// The variant costs most of its calls 1 - 4 % where it finds nothing; other launches (8 sequences of 32 K at K=1: 83.0 / 85.8) go without,
+// The variant costs most of its calls 1 - 4 % where it finds nothing (with the third copy warp 24 of 8 K at K=1 take 67.6, 20 of 16 K at K=4 122.1
+// with the search, 122.4 before there was one; NVFP4 at 32 rows 1 - 3 % and 64 rows 1 - 2 % more than then); other launches (8 sequences of 32 K at K=1: 83.0 / 85.8) go without,
 // although a table much wider than the sequences holds them back as well (8 of 2 K in one for 131 072: 117 / 29).
 // (Below eight tiles there is nothing to gain.)
-template <int D, int NT, int FMT, bool kAsync>
-cudaError_t launch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
+bool searches(const UQParams& p, const UQLaunch& x, int sms) {
   const long long max_tiles = ((long long)p.max_pages * p.PAGE + kKeys - 1) / kKeys;
-  const int bound = chunk_bound(p, x), sms = current_sms();
-  const bool pick = x.ns_eff >= 2 && bound >= 8 && 3ll * sms * bound > (long long)p.B * p.HKV * x.chunks * max_tiles;
-  return pick ? launch_as<D, NT, FMT, kAsync, true>(p, x, sms, s) : launch_as<D, NT, FMT, kAsync, false>(p, x, sms, s);
+  const int bound = chunk_bound(p, x);
+  return x.ns_eff >= 2 && bound >= 8 && 3ll * sms * bound > (long long)p.B * p.HKV * x.chunks * max_tiles;
 }
 
 }  // namespace tc
@@ -1855,40 +1855,54 @@ int uq_verify_tc_splits(const UQParams& p, const UQLaunch& x) {
 }
 
 // Largest copy unit (tokens) with which the scale slices come by the third copy warp; 0 = never, kKeys = always.  Small units mean
-// many copies per tile, and their issue becomes the kernel's pace.  GPU time without / with it in us, at up to 16 rows, 32 rows, 64 rows
-// (8 sequences of 8 K tokens; head_dim 64: 16 of 4 K; head_dim 256: 4 of 16 K on half the heads):
-//                               UltraQuant                              NVFP4
-//   head_dim 64,   16-token     42.7 / 34.0  50.1 / 40.0  57.1 / 49.2   41.7 / 33.6  49.4 / 40.6  56.8 / 48.8   (tiles of half the bytes)
-//                  32-token     35.3 / 31.0  42.4 / 39.8  49.8 / 49.1   34.0 / 30.5  41.6 / 39.3  49.5 / 48.7
-//                  64-token     32.3 / 30.4  39.4 / 39.8  48.8 / 49.2   30.9 / 29.8  38.9 / 39.5
-//                  128-token    30.9 / 30.1  39.2 / 39.9                29.6 / 29.6  38.7 / 39.5                (512-token pages the same)
-//   head_dim 128,  16-token     40.0 / 32.3  45.8 / 38.8  51.8 / 45.9   43.5 / 35.5  50.9 / 43.3  56.3 / 47.5
-//                  32-token     32.7 / 29.8  39.7 / 36.7  45.3 / 45.9   35.6 / 32.8  43.6 / 41.1  48.9 / 46.2
-//                  64-token     29.8 / 29.6
-//   head_dim 256,  16-token     39.3 / 38.9  43.4 / 42.4  50.8 / 51.6   34.4 / 36.9  40.6 / 41.8  50.3 / 50.6
-//                  32-token     37.9 / 37.5  42.4 / 42.0  50.8 / 51.2   34.8 / 37.1  40.7 / 42.1
-// At 64 rows issue slots are short: 16-token units only, although 32-token ones would gain at head_dim 64 and for NVFP4.  The copies carry no
-// cache hint: with the evict-first policy of the others they were level or up to 0.3 us slower.
-template <int D, int NT, int FMT>
+// many copies per tile, and their issue becomes the kernel's pace.  GPU time without / with it in us, at up to 16 rows, 32 rows, 64 rows;
+// short: 8 sequences of 8 K tokens (head_dim 64: 16 of 4 K; head_dim 256: 4 of 16 K on half the heads), long: 8 of 32 K (head_dim 256: 16 K).
+//                                      UltraQuant                                 NVFP4
+//   head_dim 64,   16-token   short    42.7 / 34.0   50.1 / 40.0   57.1 / 49.2    41.7 / 33.6   49.4 / 40.6   56.8 / 48.8   (tiles of half the bytes)
+//                  32-token   short    35.3 / 31.0   42.4 / 39.8   49.8 / 49.1    34.0 / 30.5   41.6 / 39.3   49.5 / 48.7
+//                             long                  114.2 / 99.0  127.3 / 119.3                114.2 / 100.4 126.9 / 121.0
+//                  64-token   short    32.3 / 30.4   39.4 / 39.8   48.8 / 49.2    30.9 / 29.8   38.9 / 39.5
+//                             long                  100.8 / 98.9  118.1 / 119.0                101.1 / 100.5 118.5 / 120.5
+//                 128-token   short    30.9 / 30.1   39.2 / 39.9                  29.6 / 29.6   38.7 / 39.5                 (512-token pages the same)
+//                             long                   96.6 / 98.9                                97.0 / 100.6
+//   head_dim 128,  16-token   short    40.0 / 32.3   45.8 / 38.8   51.8 / 45.9    43.5 / 35.5   50.9 / 43.3   56.3 / 47.5
+//                  32-token   short    32.7 / 29.8   39.7 / 36.7   45.3 / 45.9    35.6 / 32.8   43.6 / 41.1   48.9 / 46.2
+//                             long                                117.2 / 119.3                              134.5 / 122.2
+//                  64-token   long     84.2 / 80.3   95.8 / 95.7  115.6 / 119.5   94.5 / 90.6  110.4 / 110.8 120.1 / 118.7
+//       searching, 20 of 16 K         105.5 / 101.4 124.8 / 122.5                118.5 / 113.5 146.7 / 142.0 155.0 / 158.0
+//   head_dim 256,  16-token   short    39.3 / 38.9   43.4 / 42.4   50.8 / 51.6    34.4 / 36.9   40.6 / 41.8   50.3 / 50.6
+//                             long    118.5 / 118.1 128.1 / 125.3 139.7 / 141.6   96.5 / 103.6 114.2 / 119.5 137.5 / 140.9
+//                  32-token   long    115.1 / 113.4 123.9 / 122.9 139.0 / 140.4   98.1 / 105.9 116.2 / 121.3 135.0 / 141.6
+// (64-token pages at head_dim 128 without the search: what the 16-row calls would gain is not taken yet.)  Searching launches of up to 32
+// rows at head_dim 128 take it at every unit: the search's code costs their loop what the third warp gives back.  The copies carry no cache
+// hint: with the evict-first policy of the others they were level or up to 0.3 us slower.
+template <int D, int NT, int FMT, bool kPick>
 constexpr int async_unit() {
   if (D == 256) return FMT == 1 || NT == 64 ? 0 : 32;
-  if (NT == 64) return 16;
-  return D == 64 && NT == 16 ? tc::kKeys : 32;
+  if (NT == 64) return D == 64 || FMT == 1 ? 32 : 16;
+  if (D == 128) return kPick ? tc::kKeys : 32;
+  return NT == 16 ? tc::kKeys : (FMT == 1 ? 32 : 64);
+}
+
+template <int D, int NT, int FMT, bool kPick>
+static cudaError_t dispatch_copy(const UQParams& p, const UQLaunch& x, int sms, cudaStream_t s) {
+  constexpr int kUpTo = async_unit<D, NT, FMT, kPick>();
+  if constexpr (kUpTo == tc::kKeys) return tc::launch_as<D, NT, FMT, true, kPick>(p, x, sms, s);
+  else if constexpr (kUpTo == 0) return tc::launch_as<D, NT, FMT, false, kPick>(p, x, sms, s);
+  else return tc::copy_unit(p) <= kUpTo ? tc::launch_as<D, NT, FMT, true, kPick>(p, x, sms, s) : tc::launch_as<D, NT, FMT, false, kPick>(p, x, sms, s);
 }
 
 template <int D, int NT, int FMT>
-static cudaError_t dispatch_copy(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
-  constexpr int kUpTo = async_unit<D, NT, FMT>();
-  if constexpr (kUpTo == tc::kKeys) return tc::launch<D, NT, FMT, true>(p, x, s);
-  else if constexpr (kUpTo == 0) return tc::launch<D, NT, FMT, false>(p, x, s);
-  else return tc::copy_unit(p) <= kUpTo ? tc::launch<D, NT, FMT, true>(p, x, s) : tc::launch<D, NT, FMT, false>(p, x, s);
+static cudaError_t dispatch_search(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
+  const int sms = tc::current_sms();
+  return tc::searches(p, x, sms) ? dispatch_copy<D, NT, FMT, true>(p, x, sms, s) : dispatch_copy<D, NT, FMT, false>(p, x, sms, s);
 }
 
 template <int D, int FMT>
 static cudaError_t dispatch_rows(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
-  if (x.rows <= 16) return dispatch_copy<D, 16, FMT>(p, x, s);
-  if (x.rows <= 32) return dispatch_copy<D, 32, FMT>(p, x, s);
-  return dispatch_copy<D, 64, FMT>(p, x, s);
+  if (x.rows <= 16) return dispatch_search<D, 16, FMT>(p, x, s);
+  if (x.rows <= 32) return dispatch_search<D, 32, FMT>(p, x, s);
+  return dispatch_search<D, 64, FMT>(p, x, s);
 }
 
 cudaError_t uq_verify_tc_dispatch(const UQParams& p, const UQLaunch& x, cudaStream_t s) {
