@@ -157,7 +157,7 @@ def test_two_chunks_of_drafts_share_one_launch(K, HQ, HKV, D, nsplit):
 
 
 @pytest.mark.parametrize("fmt", [0, 1])
-@pytest.mark.parametrize("D,PAGE", [(64, 16), (64, 48), (64, 128), (128, 16), (128, 32), (256, 16), (256, 32)])
+@pytest.mark.parametrize("D,PAGE", [(64, 16), (64, 32), (64, 48), (64, 64), (64, 128), (128, 16), (128, 32), (256, 16), (256, 32)])
 @pytest.mark.parametrize("rows", [8, 32, 64])
 def test_scale_slices_of_small_copies_come_by_a_third_warp(D, PAGE, rows, fmt):
     """Small copy units: the scale bytes arrive 16 bytes per lane (1 .. 8 keys each, up to four pieces per lane), units past a
@@ -446,6 +446,35 @@ def test_items_cut_into_no_more_pieces_than_they_have_slots(B, HKV, long_ones, l
     assert uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
     check_close(out.float().cpu().numpy(), O.reference(qb, kc, ks, vc, vs, bt, sl), f"nsplit={nsplit}")
     assert bool((ws[n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("K", [1, 4])
+@pytest.mark.parametrize("PAGE", [64, 128, 256, 96])
+def test_searching_launches_take_the_third_copy_warp_at_every_page_size(PAGE, K, fmt):
+    """head_dim 128, up to 32 rows, few slots per item and a table wide enough for the chunk search: whole pages, 128-token parts and
+    common parts of them as copy units, scale slices 16 bytes per lane; every row against its own largest."""
+    rng = np.random.default_rng(PAGE + K)
+    B, HKV, G, D, nsplit = 40, 4, 8, 128, 3
+    sl = rng.integers(1, 300, B).astype(np.int32)
+    sl[:3] = (2100, 129, 1)
+    npg = -(-sl // PAGE)
+    pages = int(npg.sum())
+    per, kr, vr, qs = (32, (124, 128), (125, 129), 0.4) if fmt == 0 else (16, (0x28, 0x48), (0x28, 0x48), 0.3)
+    kc, vc = (rng.integers(0, 256, (pages, HKV, PAGE, D // 2), dtype=np.uint8) for _ in range(2))
+    ks, vs = (rng.integers(*r, (pages, HKV, PAGE, D // per)).astype(np.uint8) for r in (kr, vr))
+    bt, perm, at = np.zeros((B, -(-3000 // PAGE)), np.int32), rng.permutation(pages).astype(np.int32), 0
+    for b in range(B):
+        bt[b, :npg[b]] = perm[at:at + npg[b]]
+        at += npg[b]
+    qb = O.bf16_bits(qs * rng.standard_normal((B, K, HKV * G, D)).astype(np.float32))
+    ref = O.reference(qb, kc, ks, vc, vs, bt, sl) if fmt == 0 else O.reference_nvfp4(qb, kc, ks, vc, vs, bt, sl, 0.5, 0.5)
+    out = uq_cuda.uq_decode_cuda(dev(qb.view(np.int16), torch.bfloat16), *(dev(a) for a in (kc, ks, vc, vs, bt, sl)), nsplit=nsplit,
+                                 **(dict(fmt=1, k_ts=0.5, v_ts=0.5) if fmt else {}))
+    assert uq_cuda.last_path() == 2 and uq_cuda.last_status() == (0, 0, 0, 0)
+    mx = np.abs(ref).max(-1, keepdims=True)
+    mx[mx == 0] = 1
+    check_close(out.float().cpu().numpy() / mx, ref / mx, f"PAGE={PAGE}")
 
 
 CAPTURED_CHAIN = """
