@@ -122,12 +122,13 @@ UQ_DEV int group_exponent(float amax, bool paper, float c) {
 // its own kind, as ordinary launches / released before / after the wait: append of 128 tokens of 8 heads 2.9 / 3.5 / 2.6 us, of 2 048 (bulk
 // kernel) 4.4 / 5.9 / 4.0, NVFP4 of 200 tokens 3.1 / 4.2 / 2.8, rotation of 2 048 rows 3.0 / 4.3 / 2.5; 64 new tokens and the verify call
 // behind them 30.8 / 28.5 / 28.4 (28.9 with no early release). An early release pays while the next grid finds room beside
-// this one, or when this one takes several waves and the release comes with its last: bulk appends between the two bounds below (NVFP4, 77
-// registers: two grids of 444 blocks fit, one of 888) let go at their end - 2 048 NVFP4 tokens, 512 blocks, 6.7 us released early, 5.5 at the end;
-// 32 768 tokens 52.4 and 52.6.  The per-row kernel releases early at all its sizes for the verify call behind it (200 tokens and that call
+// this one, or when this one takes several waves: its last blocks start, and with them the release is complete, when what came before is long
+// over, so it may as well come first (12 289 NVFP4 tokens, 3 072 blocks, 23.3 us, 23.5 after the wait).  Bulk appends between the two bounds
+// below (NVFP4, 77 registers: two grids of 444 blocks fit, one of 888) let go at their end - 2 048 NVFP4 tokens, 512 blocks, 6.7 us released
+// early, 5.5 at the end.  The per-row kernel releases early at all its sizes for the verify call behind it (200 tokens and that call
 // 29.6, 30.0 at the end), although a chain of 200 to 255 tokens' appends alone would be quicker without (3.9 / 2.8).
 constexpr unsigned kReleaseUpTo = 384, kReleaseFrom = 2048;
-UQ_DEV bool bulk_releases_early() { const unsigned blocks = gridDim.x * gridDim.y; return blocks <= kReleaseUpTo || blocks >= kReleaseFrom; }
+UQ_DEV unsigned bulk_blocks() { return gridDim.x * gridDim.y; }
 
 // e2m1 code of y = x / 2^e: nearest of {0,.5,1,1.5,2,3,4,6}, ties to the smaller magnitude (the
 // reference's first-index argmin), sign bit from (y < 0) whatever the magnitude.
@@ -362,8 +363,9 @@ __global__ void __launch_bounds__(256) uq_append_bulk_kernel(uint8_t* __restrict
                                                              uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                              const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
                                                              int PAGE, int page_shift, int paper, float c, int pdl) {
+  if (pdl && bulk_blocks() >= kReleaseFrom) uq_pdl_release();
   const unsigned tid = uq_pdl_wait_index();
-  if (pdl && bulk_releases_early()) uq_pdl_release();
+  if (pdl && bulk_blocks() <= kReleaseUpTo) uq_pdl_release();
   constexpr bool kExactTies = sizeof(T) == 4;   // fp32 inputs can sit anywhere: half-way values are corrected by comparison
   constexpr int NP = bulk_pieces<T>();          // pieces per thread: 128 bytes of input in flight
   const int stream = blockIdx.y;
@@ -582,8 +584,9 @@ __global__ void __launch_bounds__(256) uq_append_nvfp4_bulk_kernel(uint8_t* __re
                                                                    uint8_t* __restrict__ vs, const T* __restrict__ key, const T* __restrict__ value,
                                                                    const int64_t* __restrict__ slots, uint32_t np, int HKV, uint32_t hkv_magic, int D,
                                                                    int PAGE, int page_shift, float k_ts, float v_ts, int pdl) {
+  if (pdl && bulk_blocks() >= kReleaseFrom) uq_pdl_release();
   const unsigned tid = uq_pdl_wait_index();
-  if (pdl && bulk_releases_early()) uq_pdl_release();
+  if (pdl && bulk_blocks() <= kReleaseUpTo) uq_pdl_release();
   constexpr int NP = bulk_pieces<T>();
   constexpr bool kAddZero = sizeof(T) == 4;   // fp32 inputs: any product can underflow, +0 is added after the multiplication
   // a 16-bit input's smallest non-zero magnitude (2^-133 bf16, 2^-24 fp16) times the reciprocal stays a normal number

@@ -45,9 +45,12 @@ def test_indexes_of_read_only_loads_come_out_of_the_wait():
 
 
 def test_appends_release_their_successors_after_their_own_wait():
-    """Before it, a waiting kernel would let the next one in, and that one the next: a pile of waiting grids in the working one's way."""
+    """Before it, a waiting kernel would let the next one in, and that one the next: a pile of waiting grids in the working one's way.
+    Only a grid of several waves, whose last blocks start late, may release first."""
     for name, body in kernels("uq_append.cu").items():
-        assert body.count("uq_pdl_release()") == 1 and body.index("uq_pdl_release()") > body.index("uq_pdl_wait_index()"), name
+        wait = body.index("uq_pdl_wait_index()")
+        first = "if (pdl && bulk_blocks() >= kReleaseFrom) uq_pdl_release();" in body[:wait]
+        assert first == ("bulk" in name) and body[:wait].count("uq_pdl_release()") == first and body[wait:].count("uq_pdl_release()") == 1, name
 
 
 def test_no_multiprocessor_count_is_written_down():
