@@ -145,15 +145,16 @@ def _need_cuda(*ts):
 def _params(q, kc, ks, vc, vs, bt, sl, nsplit, sm_scale, variant=0, mb=0, fmt=0, k_ts=1.0, v_ts=1.0):
     B, K, HQ, D = q.shape
     kshape = kc.shape
-    # the structure's fields in its order, packed at once (a store per field is half of the call's arithmetic)
-    v = (q.data_ptr(), kc.data_ptr(), ks.data_ptr(), vc.data_ptr(), vs.data_ptr(), bt.data_ptr(), sl.data_ptr(), 0, 0, 0, B, K, HQ, kshape[1], D, kshape[2],
-         bt.shape[1], int(nsplit), float(sm_scale), int(variant), int(mb), int(fmt), float(k_ts), float(v_ts))
-    try:
-        return UQParams.from_buffer_copy(_PARAMS.pack(*v))
+    try:   # the structure's fields in its order, packed at once (a store per field is half of the call's arithmetic)
+        return UQParams.from_buffer_copy(_PARAMS.pack(q.data_ptr(), kc.data_ptr(), ks.data_ptr(), vc.data_ptr(), vs.data_ptr(), bt.data_ptr(), sl.data_ptr(),
+                                                      0, 0, 0, B, K, HQ, kshape[1], D, kshape[2], bt.shape[1], int(nsplit), float(sm_scale), int(variant),
+                                                      int(mb), int(fmt), float(k_ts), float(v_ts)))
     except (struct.error, OverflowError):   # an integer beyond 32 bits, a scale beyond fp32: as a store makes them (truncated, infinite)
         p = UQParams()
-        for (name, _), x in zip(UQParams._fields_, v):
-            setattr(p, name, x)
+        p.q, p.kc, p.ks, p.vc, p.vs = q.data_ptr(), kc.data_ptr(), ks.data_ptr(), vc.data_ptr(), vs.data_ptr()
+        p.block_table, p.seq_lens = bt.data_ptr(), sl.data_ptr()
+        p.B, p.K, p.HQ, p.HKV, p.D, p.PAGE, p.max_pages, p.nsplit = B, K, HQ, kshape[1], D, kshape[2], bt.shape[1], int(nsplit)
+        p.sm_scale, p.variant, p.mb, p.fmt, p.k_ts, p.v_ts = float(sm_scale), int(variant), int(mb), int(fmt), float(k_ts), float(v_ts)
         return p
 
 
